@@ -61,3 +61,63 @@ def test_one_part_and_bad_k(ctx):
     with pytest.raises(tc.TCError) as e:
         ctx.parts_lp(ug, 65)
     assert e.value.code == "TC_E_INVALID"
+
+
+def _mix(x):
+    with np.errstate(over="ignore"):
+        x = x + np.uint64(0x9E3779B97F4A7C15)
+        x = (x ^ (x >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        x = (x ^ (x >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return x ^ (x >> np.uint64(31))
+
+
+def _hash(seed, it, v, l):
+    return _mix(np.uint64(seed) ^ _mix((np.uint64(it) << np.uint64(40)) ^ (v.astype(np.uint64) << np.uint64(8)) ^
+                                       l.astype(np.uint64))) >> np.uint64(32)
+
+
+def lp_reference(rp, col, k, seed, iterations):
+    """The label propagation of tc_partition.cu restated in numpy."""
+    n = len(rp) - 1
+    v = np.arange(n)
+    label = v * k // n
+    rows = np.repeat(v, np.diff(rp))
+    cap = (n * 103 + 100 * k - 1) // (100 * k)
+    for it in range(iterations if k > 1 else 0):
+        count = np.zeros((n, k), np.int64)
+        np.add.at(count, (rows, label[col]), 1)
+        tie = np.stack([_hash(seed, it, v, np.full(n, l)) >> np.uint64(1) for l in range(k)], 1).astype(np.int64)
+        tie[v, label] = 0xFFFFFFFF
+        key = (count << 32) | tie
+        key[count == 0] = 0
+        best = key.argmax(1)
+        wish = np.where((key.max(1) == 0) | (best == label), -1, best)
+        cand = wish >= 0
+        flow = np.zeros((k, k), np.int64)
+        np.add.at(flow, (label[cand], wish[cand]), 1)
+        want = flow.sum(0)
+        room0 = np.maximum(0, cap - np.bincount(label, minlength=k))
+        leave = [sum(int(f if room0[t] >= want[t] else f * room0[t] // want[t]) for t, f in enumerate(flow[b]) if f)
+                 for b in range(k)]
+        room = room0 + np.array(leave)
+        h = _hash(seed ^ 0x5A5A5A5A, it, v, np.maximum(wish, 0))
+        go = cand & (h * want[wish].astype(np.uint64) < (room[wish].astype(np.uint64) << np.uint64(32)))
+        label = np.where(go, wish, label)
+        if go.sum() * 1000 < n:
+            break
+    return label.astype(np.int32)
+
+
+@pytest.mark.parametrize("k", [1, 2, 7, 8, 9, 16, 17, 33, 64])
+@pytest.mark.parametrize("iterations", [0, 1, 8, 9, 30])
+def test_parts_equal_the_restatement(ctx, k, iterations):
+    """Part counts around the packed counters' sizes, iterations around a batch,
+    degrees around the group (255), warp (1024) and block paths, isolated ids."""
+    src, dst = gen.rmat(11, 8)
+    n = 5000
+    hub = np.concatenate([np.full(d, 4000 + i) for i, d in enumerate((255, 256, 257, 1023, 1024, 1025, 3500))])
+    leaf = np.concatenate([np.arange(d) for d in (255, 256, 257, 1023, 1024, 1025, 3500)])
+    rp, col = oracle.clean(np.concatenate((src, hub)), np.concatenate((dst, leaf)), n)
+    ug = ctx.upload_ugraph(rp, col)
+    got = ctx.parts_lp(ug, k, seed=77, iterations=iterations)
+    assert np.array_equal(got, lp_reference(rp, col, k, 77, iterations))
