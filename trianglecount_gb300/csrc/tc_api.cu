@@ -17,6 +17,10 @@ thread_local std::string g_last_error;
 
 constexpr int kVersion = 10000;  // 1.0.0
 
+// Graphs counted in one launch: see single_count.
+constexpr int64_t kSingleMinRows = 64, kSingleMaxEdges = 1 << 18, kSingleMaxSkewed = 1 << 14;
+constexpr int32_t kSingleMaxDeg = 64;
+
 // ---- CSR validation (rows strictly ascending, ids in range) ----
 struct ValidateErr {
     int code;     // 0 ok, 1 row_ptr, 2 id range, 3 order
@@ -168,6 +172,8 @@ int check_graph(const tc_graph *g) {
     return TC_OK;
 }
 
+bool packed_graph(const tc_graph *g);
+
 // Count scratch of a graph: descriptor, work words + result, CountScratch.
 int ensure_count_scratch(tc_graph *g) {
     tc_ctx *ctx = g->ctx;
@@ -179,15 +185,15 @@ int ensure_count_scratch(tc_graph *g) {
     }
     if (!g->d_desc) {  // the flat count needs only the work words
         TC_TRY(dalloc((void **)&g->d_desc, sizeof(GraphDesc), ctx->stream));
-        TC_TRY(scratch_alloc(&g->sc, g->n_rows + 1, g->nnz,
-                             std::min(g->n_rows, g->nnz) + 1, ctx->stream));
     }
+    TC_TRY(scratch_alloc(&g->sc, g->n_rows + 1, g->nnz, std::min(g->n_rows, g->nnz) + 1, 1, packed_graph(g),
+                         ctx->stream));
     return TC_OK;
 }
 
 __global__ void set_desc_kernel(GraphDesc *dst, GraphDesc d) { *dst = d; }
 
-// Up to eight descriptors as one kernel parameter (512 bytes): a table is
+// Up to eight descriptors as one kernel parameter (576 bytes): a table is
 // written in stream order with no host copy (a copy from pageable memory
 // would first wait for the stream to drain).
 struct DescBlock {
@@ -226,8 +232,8 @@ void capture_count(tc_graph *g, unsigned long long *res) {
         return;
     }
     int nl = 0;
-    const int st = launch_count(g->d_desc, 1, (g->n_rows + 31) / 32, g->n_rows + 1, g->n_rows, g->sc, g->d_work, res,
-                                false, ctx->tuned, s, &nl, ctx->kev, g->n_roots < g->n_rows);
+    const int st = launch_count(g->d_desc, 1, (g->n_rows + 31) / 32, g->n_rows + 1, g->nnz,
+                                packed_graph(g), g->n_rows, g->sc, g->d_work, res, false, ctx->tuned, s, &nl, ctx->kev, g->n_roots < g->n_rows);
     cudaGraph_t graph = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(s, &graph);
     cudaGraphExec_t exec = nullptr;
@@ -243,13 +249,42 @@ void capture_count(tc_graph *g, unsigned long long *res) {
 
 bool flat_count(const tc_graph *g) { return g->max_deg >= 0 && g->max_deg <= g->ctx->tuned.flat_max_deg; }
 
+// The packed count serves launches whose graphs are skewed (their longest row,
+// where it is known, above kSkew x the mean) or small enough that most ids are
+// low blocks'.  Without hubs the entries hold one id each and lie in the high
+// blocks, whose hashes cost more than the plain-id tables: Erdos-Renyi n = 1 M of
+// mean degree 8 / 40, longest rows 3.3 / 2.4 x the mean, 0.25 / 1.37 ms there,
+// 0.37 / 1.6 packed; n = 30 K of mean degree 40 0.18 and 0.16.  (R-MAT and
+// Chung-Lu graphs of the same sizes have 6 to 60 x the mean.)
+constexpr int64_t kSkew = 5, kPackRows = 61440;
+bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
+    if (!packed_count(tn)) return false;
+    int64_t V = 0, E = 0, gain = 0;
+    for (int i = 0; i < n; ++i) {
+        const tc_graph *g = gs[i];
+        if (g->max_deg < 0 || g->n_rows <= kPackRows || g->max_deg * g->n_rows > kSkew * g->nnz) gain += g->nnz;
+        V += g->n_rows + 1;
+        E += g->nnz;
+    }
+    return 2 * gain >= E && pack_fits(V, E);
+}
+bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
+
+// A graph of few edges that no lane-per-root count takes is counted by one
+// launch on its own ids (launch_single).
+bool single_count(const tc_graph *g) {
+    const Tuned &tn = g->ctx->tuned;
+    return packed_count(tn) && tn.flat_max_deg > 0 && !flat_count(g) && g->n_rows >= kSingleMinRows &&
+           g->nnz <= (g->max_deg >= 0 && g->max_deg <= kSingleMaxDeg ? kSingleMaxEdges : kSingleMaxSkewed);
+}
+
 // Everything a count of g needs before its launches: the work words, the
 // scratch and the descriptor, and -- from the graph's second chain count on
 // -- the captured chain.  Callers that time a count run this before their
 // start event, so neither allocations nor a capture land in the timed span.
 int prepare_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long long *results) {
     tc_ctx *ctx = g->ctx;
-    if (flat_count(g)) {  // every list fits a lane's registers: one kernel, no transpose or hash tables
+    if (flat_count(g) || single_count(g)) {  // one kernel, no scratch
         if (!g->d_work) {
             void *p = nullptr;
             TC_TRY(dalloc(&p, sizeof(CountWork) + sizeof(unsigned long long), ctx->stream));
@@ -265,6 +300,7 @@ int prepare_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long
     d.col = g->col;
     d.n_rows = g->n_rows;
     d.n_roots = g->n_roots;
+    d.mbits = pack_mask_bits(g->n_rows);
     d.chunk_base = 0;
     d.vbase = 0;
     d.per_root = per_root;
@@ -303,6 +339,17 @@ int enqueue_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long
         return launch_flat(g->rp, g->col, g->n_roots, g->max_deg, g->d_work, res, per_root, ctx->tuned, ctx->stream,
                            launches, ctx->kev);
     }
+    if (single_count(g)) {
+        ctx->kev_recorded = true;
+        GraphDesc d;
+        memset(&d, 0, sizeof d);
+        d.rp = g->rp;
+        d.col = g->col;
+        d.n_rows = g->n_rows;
+        d.n_roots = g->n_roots;
+        d.per_root = per_root;
+        return launch_single(d, g->d_work, res, ctx->tuned, ctx->stream, launches, ctx->kev);
+    }
     const int64_t chunks = (g->n_rows + 31) / 32;
     ctx->kev_recorded = chunks > 0;
     ++g->chain_counts;
@@ -313,7 +360,7 @@ int enqueue_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long
         if (launches) *launches = g->exec_launches;
         return TC_OK;
     }
-    return launch_count(g->d_desc, 1, chunks, g->n_rows + 1, g->n_rows, g->sc, g->d_work, res, per_root != nullptr,
+    return launch_count(g->d_desc, 1, chunks, g->n_rows + 1, g->nnz, packed_graph(g), g->n_rows, g->sc, g->d_work, res, per_root != nullptr,
                         ctx->tuned, ctx->stream, launches, ctx->kev, g->n_roots < g->n_rows);
 }
 
@@ -393,13 +440,16 @@ void ctx_release(tc_ctx *c) {
     delete c;
 }
 
-int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, cudaStream_t s) {
+int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool packed,
+                  cudaStream_t s) {
     // in-list offsets and slots are int32 over the launch's pooled edges
     if (E >= INT32_MAX)
         return set_error(TC_E_RANGE,
                          "one count launch holds fewer than 2^31 - 1 oriented edges in total, got %lld: split the "
                          "batch",
                          (long long)E);
+    if (packed) return sc->pk.units ? TC_OK : pack_scratch_alloc(&sc->pk, V, E, n_graphs, s);
+    if (sc->mid) return TC_OK;
     sc->heavy_cap = heavy_cap;
     TC_TRY(dalloc((void **)&sc->heavy, sizeof(HeavyEntry) * (size_t)std::max<int64_t>(heavy_cap, 1), s));
     TC_TRY(dalloc((void **)&sc->light_list, sizeof(uint32_t) * (size_t)std::max<int64_t>(V, 1), s));
@@ -421,6 +471,7 @@ void scratch_free(CountScratch *sc, cudaStream_t s) {
     dfree(sc->out_work, s);
     dfree(sc->in_list, s);
     dfree(sc->mid, s);
+    pack_scratch_free(&sc->pk, s);
     *sc = CountScratch();
 }
 
@@ -464,6 +515,7 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
         desc[(size_t)i].col = g->col;
         desc[(size_t)i].n_rows = g->n_rows;
         desc[(size_t)i].n_roots = g->n_roots;
+        desc[(size_t)i].mbits = pack_mask_bits(g->n_rows);
         desc[(size_t)i].chunk_base = chunks;
         desc[(size_t)i].vbase = vtot;
         desc[(size_t)i].ebase = etot;
@@ -472,6 +524,7 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
+    const bool packed = packed_graphs(graphs, n, ctx->tuned);
     CountScratch sc;
     DBuf<GraphDesc> d_desc;
     DBuf<unsigned char> d_work;
@@ -486,13 +539,13 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
     }
     int st = d_desc.alloc((size_t)n, s);
     if (st == TC_OK) st = d_work.alloc(out_bytes, s);
-    if (st == TC_OK) st = scratch_alloc(&sc, vtot, etot, cap, s);
+    if (st == TC_OK) st = scratch_alloc(&sc, vtot, etot, cap, n, packed, s);
     if (st == TC_OK && cudaMemcpyAsync(d_desc.p, desc.data(), sizeof(GraphDesc) * (size_t)n, cudaMemcpyHostToDevice,
                                        s) != cudaSuccess)
         st = set_error(TC_E_CUDA, "descriptor upload failed");
     if (st == TC_OK && cudaEventRecord(ctx->ev[0], s) != cudaSuccess) st = set_error(TC_E_CUDA, "event record failed");
     if (st == TC_OK)
-        st = launch_count(d_desc.p, n, chunks, vtot, max_rows, sc, (CountWork *)d_work.p,
+        st = launch_count(d_desc.p, n, chunks, vtot, etot, packed, max_rows, sc, (CountWork *)d_work.p,
                           (unsigned long long *)(d_work.p + sizeof(CountWork)), false, ctx->tuned, s, nullptr, nullptr,
                           halo_parts);
     if (st == TC_OK && cudaEventRecord(ctx->ev[1], s) != cudaSuccess) st = set_error(TC_E_CUDA, "event record failed");
@@ -887,13 +940,17 @@ int tc_count_per_root(tc_ctx *ctx, tc_graph *g, uint64_t *per_root, uint64_t *to
     if (g->n_roots)
         TC_CUDA(cudaMemcpyAsync(per_root, pr.p, sizeof(unsigned long long) * (size_t)g->n_roots,
                                 cudaMemcpyDeviceToHost, s));
-    TC_CUDA(cudaMemcpyAsync(ctx->h_pinned, g->d_work, sizeof(CountWork), cudaMemcpyDeviceToHost, s));
+    TC_CUDA(cudaMemcpyAsync(ctx->h_pinned, g->d_work, sizeof(CountWork) + sizeof(unsigned long long),
+                            cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaStreamSynchronize(s));
     if (((const CountWork *)ctx->h_pinned)->error)
         return set_error(TC_E_STATE, "%s", count_error_text(((const CountWork *)ctx->h_pinned)->error));
     if (total) {
-        uint64_t t = 0;
-        for (int64_t u = 0; u < g->n_roots; ++u) t += per_root[u];
+        // the one-kernel counts and the packed count sum the hits beside the
+        // per-root counts; the plain-id tables credit the roots only
+        const bool summed = flat_count(g) || single_count(g) || packed_graph(g);
+        uint64_t t = summed ? *(const unsigned long long *)((const CountWork *)ctx->h_pinned + 1) : 0;
+        for (int64_t u = 0; u < g->n_roots && !summed; ++u) t += per_root[u];
         *total = t;
     }
     return TC_OK;
@@ -979,6 +1036,7 @@ int tc_batch_create(tc_ctx *ctx, tc_graph *const *graphs, int n, tc_batch **out)
         desc[i].col = g->col;
         desc[i].n_rows = g->n_rows;
         desc[i].n_roots = g->n_roots;
+        desc[i].mbits = pack_mask_bits(g->n_rows);
         desc[i].chunk_base = chunks;
         desc[i].vbase = vtot;
         desc[i].ebase = etot;
@@ -988,10 +1046,11 @@ int tc_batch_create(tc_ctx *ctx, tc_graph *const *graphs, int n, tc_batch **out)
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
+    const bool packed = packed_graphs(graphs, n, ctx->tuned);
     b->total_chunks = chunks;
     b->total_vertices = vtot;
     int st = dalloc((void **)&b->d_desc, sizeof(GraphDesc) * (size_t)n, s);
-    if (st == TC_OK) st = scratch_alloc(&b->sc, vtot, etot, cap, s);
+    if (st == TC_OK) st = scratch_alloc(&b->sc, vtot, etot, cap, n, packed, s);
     if (st == TC_OK) st = dalloc((void **)&b->d_work, sizeof(CountWork) + sizeof(unsigned long long) * (size_t)n, s);
     if (st == TC_OK && cudaMallocHost(&b->h_out, sizeof(CountWork) + sizeof(unsigned long long) * (size_t)n) != cudaSuccess)
         st = set_error(TC_E_NOMEM, "pinned result buffer");
@@ -1005,7 +1064,7 @@ int tc_batch_create(tc_ctx *ctx, tc_graph *const *graphs, int n, tc_batch **out)
     if (st == TC_OK && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         st = set_error(TC_E_CUDA, "stream capture could not start");
     if (st == TC_OK) {
-        int ls = launch_count(b->d_desc, n, chunks, vtot, max_rows, b->sc, b->d_work,
+        int ls = launch_count(b->d_desc, n, chunks, vtot, etot, packed, max_rows, b->sc, b->d_work,
                               (unsigned long long *)(b->d_work + 1), false, ctx->tuned, s, &b->launches, b->kev,
                               halo_parts);
         cudaError_t e = cudaStreamEndCapture(s, &b->graph);
@@ -1076,6 +1135,7 @@ int enqueue_group_count(tc_ctx *ctx, tc_graph *const *gs, int n, unsigned long l
         d.col = g->col;
         d.n_rows = g->n_rows;
         d.n_roots = g->n_roots;
+        d.mbits = pack_mask_bits(g->n_rows);
         d.chunk_base = chunks;
         d.vbase = vtot;
         d.ebase = etot;
@@ -1084,10 +1144,11 @@ int enqueue_group_count(tc_ctx *ctx, tc_graph *const *gs, int n, unsigned long l
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
+    const bool packed = packed_graphs(gs, n, ctx->tuned);
     grp->s = s;
     TC_TRY(grp->desc.alloc((size_t)n, s));
     TC_TRY(grp->work.alloc(1, s));
-    TC_TRY(scratch_alloc(&grp->sc, vtot, etot, cap, s));
+    TC_TRY(scratch_alloc(&grp->sc, vtot, etot, cap, n, packed, s));
     for (int i0 = 0; i0 < n; i0 += 8) {
         DescBlock blk;
         const int m = std::min(8, n - i0);
@@ -1095,7 +1156,7 @@ int enqueue_group_count(tc_ctx *ctx, tc_graph *const *gs, int n, unsigned long l
         set_descs_kernel<<<1, 8, 0, s>>>(grp->desc.p + i0, blk, m);
         TC_CUDA(cudaGetLastError());
     }
-    return launch_count(grp->desc.p, n, chunks, vtot, max_rows, grp->sc, grp->work.p, d_res, false, ctx->tuned, s,
+    return launch_count(grp->desc.p, n, chunks, vtot, etot, packed, max_rows, grp->sc, grp->work.p, d_res, false, ctx->tuned, s,
                         nullptr, nullptr, halo_parts);
 }
 

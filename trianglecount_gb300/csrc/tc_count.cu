@@ -1548,6 +1548,7 @@ int resolve_tuning(const tc_tuning &t, int sm_count, Tuned *out) {
     if (occ < 1) return set_error(TC_E_INVALID, "count kernel does not fit on an SM with %zu B shared memory", r.smem);
     const int bps = t.blocks_per_sm > 0 ? std::min(t.blocks_per_sm, occ) : occ;
     r.blocks = sm_count * bps;
+    TC_TRY(pack_blocks(sm_count, t.blocks_per_sm, &r.pack_blocks));
     // The auxiliary kernels walk the 32-row chunks grid-stride.  With no more
     // blocks than fit on the GPU at once, the chunks in flight form one moving
     // window, so a batch touches its graphs (and their in-lists) one after the
@@ -1572,10 +1573,7 @@ static int scan_launches(int64_t n) {
     return n <= kScanTile ? 1 : 2 + scan_launches((n + kScanTile - 1) / kScanTile);
 }
 
-// Records a kernel-timing event on s; inside a stream capture (the plain
-// count's cached graph) as an external event node, so that every replay of
-// the captured chain records it too.
-static int record_kernel_event(cudaEvent_t ev, cudaStream_t s) {
+int record_kernel_event(cudaEvent_t ev, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     TC_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs == cudaStreamCaptureStatusActive) TC_CUDA(cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal));
@@ -1584,8 +1582,12 @@ static int record_kernel_event(cudaEvent_t ev, cudaStream_t s) {
 }
 
 int launch_count(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, int64_t total_vertices,
-                 int64_t max_rows, const CountScratch &sc, CountWork *work, unsigned long long *results, bool per_root,
-                 const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev, bool halo_parts) {
+                 int64_t total_edges, bool packed, int64_t max_rows, const CountScratch &sc, CountWork *work,
+                 unsigned long long *results, bool per_root, const Tuned &tn, cudaStream_t s, int *launches,
+                 cudaEvent_t *kev, bool halo_parts) {
+    if (packed)
+        return launch_packed(d_desc, n_graphs, total_chunks, total_vertices, total_edges, sc.pk, work, results, per_root, tn,
+                             s, launches, kev);
     KParams P;
     P.gd = d_desc;
     P.n_graphs = n_graphs;

@@ -73,10 +73,21 @@ struct GraphDesc {
     int64_t vbase;                // exclusive prefix of (n_rows + 1) over graphs
     int64_t ebase;                // exclusive prefix of nnz over graphs
     unsigned long long *per_root; // optional g_sum output (zeroed by the caller)
+    int32_t mbits;                // mask bits of the packed rows' entries (pack_mask_bits)
 };
 
 struct HeavyEntry {
     int32_t g, u, unit_base, n_slices;  // units = ceil(d+(u) / tile) * n_slices
+};
+
+// The packed count's arrays (tc_pack.cu), pooled over a launch's graphs:
+// V = sum (n_rows + 1), E = sum nnz.
+struct PackScratch {
+    uint32_t *code = nullptr;      // V, then 512 words per graph (popularity histogram and cursors)
+    int4 *desc = nullptr;          // V
+    uint4 *ent = nullptr;          // (E + 13 V) / 4 + 2
+    uint32_t *mid_list = nullptr;  // E / 33 + 1
+    uint2 *units = nullptr;        // E / 16 + 1
 };
 
 // Device arrays of one count launch, sized for its graphs (pooled over a batch):
@@ -92,8 +103,11 @@ struct CountScratch {
     unsigned long long *out_work = nullptr; // V
     int32_t *in_list = nullptr;             // E
     uint8_t *mid = nullptr;                 // E: edge done middle-centric
+    PackScratch pk;                         // the packed count's arrays instead of the above
 };
-int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, cudaStream_t s);
+// Allocates the arrays of the packed or the plain-id count, where sc does not have them yet.
+int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool packed,
+                  cudaStream_t s);
 void scratch_free(CountScratch *sc, cudaStream_t s);
 
 // Per-launch device words, zeroed by one memset before each count.
@@ -102,6 +116,7 @@ struct CountWork {
     unsigned int heavy_cursor;
     unsigned int small_cursor;       // light-task cursor
     unsigned int aux_cursor[2];      // chunk cursors of in_count, transpose/classify
+    unsigned int self_loops;         // the packed count met a row that is its own member
     int error;                       // 1: heavy-unit list overflow; 2: a bulk-copy staging wait gave up
     unsigned long long total_work;   // sum over oriented edges of the cheaper side's length
     unsigned long long n_tasks;      // tasks listed by the classifier, one atomic per chunk for both
@@ -126,11 +141,35 @@ struct Tuned {  // resolved tc_tuning with derived table geometry
     int log_block_slots;
     int threads;         // per block
     int blocks;          // persistent grid
+    int pack_blocks;     // persistent grid of the packed count
     int aux_blocks;      // resident grid of the per-chunk auxiliary kernels
     size_t smem;         // dynamic shared memory bytes
 };
 
 int resolve_tuning(const tc_tuning &t, int sm_count, Tuned *out);
+
+// ---- packed count (tc_pack.cu) ----------------------------------------------------
+// The default tuning's count of skewed graphs (packed_graphs); the options that name a table form (linear
+// probing, pair tables, id bitmaps, sorted lists) count on tc_count.cu's tables
+// of plain ids.
+inline bool packed_count(const Tuned &tn) {
+    return tn.probe_kicks > 0 && !tn.hash_pairs && !tn.heavy_bitmap && tn.intersect == 0;
+}
+bool pack_fits(int64_t V, int64_t E);  // else the plain-id tables count it
+int pack_mask_bits(int64_t n_rows);
+int pack_scratch_alloc(PackScratch *ps, int64_t V, int64_t E, int n_graphs, cudaStream_t s);
+void pack_scratch_free(PackScratch *ps, cudaStream_t s);
+int pack_blocks(int sm_count, int blocks_per_sm, int *out);
+int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, int64_t total_vertices,
+                  int64_t total_edges, const PackScratch &ps, CountWork *work, unsigned long long *results,
+                  bool per_root, const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev);
+// One-kernel count of a graph of few edges, on its own ids.
+int launch_single(const GraphDesc &d, CountWork *work, unsigned long long *result, const Tuned &tn, cudaStream_t s,
+                  int *launches, cudaEvent_t *kev);
+// Records a kernel-timing event on s; inside a stream capture (the plain
+// count's cached graph) as an external event node, so that every replay of
+// the captured chain records it too.
+int record_kernel_event(cudaEvent_t ev, cudaStream_t s);
 
 // launch_count for callers that cannot allocate: the in-edge scan keeps its
 // tile sums in scan_tmp (scan_tmp_cap values); nothing is allocated.
@@ -153,7 +192,7 @@ int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_
 // of the launch is a halo part (n_roots < n_rows); its heavy units then run
 // the count kernel's instance for small units.
 int launch_count(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, int64_t total_vertices,
-                 int64_t max_rows, const CountScratch &sc, CountWork *work, unsigned long long *results, bool per_root,
+                 int64_t total_edges, bool packed, int64_t max_rows, const CountScratch &sc, CountWork *work, unsigned long long *results, bool per_root,
                  const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev = nullptr,
                  bool halo_parts = false);
 
