@@ -70,7 +70,7 @@ constexpr int kWarpTile = 96, kBlockTile = 768;     // high entries of a root lo
 constexpr int kWarpWords = kLow / 2 + (1 << kLogWarpH);
 constexpr int kBlockWords = kLow / 2 + (1 << kLogBlockH);
 static_assert(kBlockWords <= kWarps * kWarpWords, "the block table lies in the warps' tables");
-constexpr int kPiece = 1 << (kLogWarpH - 1);        // members of a long row that pack hashes at a time
+constexpr int kPiece = 128, kSmallScan = 512;       // see pack_kernel
 
 // Where a row's entries lie: quads of four entries (16 bytes, zero-padded), the
 // high blocks' first, then the low blocks' in pairs of quads (octets).  Row x of
@@ -280,22 +280,24 @@ __global__ void __launch_bounds__(kThreads) assign_kernel(PackParams P) {
     }
 }
 
-// Rows to entries, one warp per 32-row chunk.  Rows of at most 32 members:
-// whole rows are laid side by side in windows of at most 32 members, one lane
-// each, and the lanes of one row with one block merge their bits
-// (__match_any_sync).  Longer rows: the warp ORs the members' bits into a
-// table by block (16-bit masks for the lowest blocks, a hash of entries for
-// the rest) and writes the non-empty places in order, so the low blocks
-// mostly ascend.  A row of more than kPiece members hashes its high blocks
-// kPiece members at a time; a high block may then have several entries with
-// different bits, which neither the streaming nor the hashes (filled by OR)
-// mind.
+// Rows to entries, a warp for pack_rows rows.  Rows of at most 32 members: whole
+// rows are laid side by side in windows of at most 32 members, one lane each,
+// and the lanes of one row with one block merge their bits (__match_any_sync).
+// Longer rows, kPiece members at a time: the low blocks' bits are ORed into masks
+// by block, the high ones go out as they are (their blocks, without hubs, seldom
+// meet: hashing them to merge their bits cost more than the whole row's other
+// work, R-MAT 23's eight parts 10.1 ms of packing, 6.4 without).  Then the masks
+// are scanned in order and the non-empty ones dealt out, so that the entries
+// ascend; a row of at most kPiece members scans the first kSmallScan blocks and
+// lists the others as it meets them, since scanning 2048 blocks for 100 members
+// would be most of its work.
 __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
-    __shared__ __align__(16) uint32_t s_tab[kWarps][kWarpWords];
+    __shared__ __align__(16) uint32_t s_dir[kWarps][kLow / 2];
+    __shared__ uint16_t s_list[kWarps][kPiece];
     __shared__ int4 s_row[kWarps][kWarp];
     const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-    uint32_t *dir = s_tab[warp], *hs = dir + kLow / 2;
-    for (int i = lane; i < kWarpWords; i += kWarp) dir[i] = 0;
+    uint32_t *dir = s_dir[warp];
+    for (int i = lane; i < kLow / 2; i += kWarp) dir[i] = 0;
     __syncwarp();
     const uint32_t le = kFull >> (31 - lane), lt = le >> 1;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
@@ -381,10 +383,8 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
             const uint32_t rx = (uint32_t)__shfl_sync(kFull, (int)x, k);
             uint32_t *out = reinterpret_cast<uint32_t *>(P.ent + rq);
             const bool small = rd <= kPiece;
-            const int lg = small ? max(7, 33 - __clz(rd - 1)) : kLogWarpH;  // places: twice the members, rounded up
-            const int hn = 1 << lg;
-            const int dn = small ? hn : kLow;  // masks kept by block; a small row's other low blocks are hashed
-            int o = 0, nl = 0;  // high entries written; low blocks met first by this lane
+            const int dn = small ? kSmallScan : kLow;  // blocks scanned in order; a small row lists its others
+            int o = 0, nl = 0, n_list = 0;  // high entries written; low blocks of this lane; blocks listed
             for (int p0 = 0; p0 < rd; p0 += kPiece) {
                 const int p1 = min(rd, p0 + kPiece);
                 uint32_t e[kPiece / kWarp];
@@ -400,43 +400,28 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
                 }
 #pragma unroll
                 for (int q = 0; q < kPiece / kWarp; ++q) {
-                    if (!e[q]) continue;
-                    const bool low = e[q] < kLowEnd;
-                    const int sh = low ? 16 : mb;
-                    const uint32_t blk = e[q] >> sh;
-                    if (blk < (uint32_t)dn) {
+                    if (p0 + q * kWarp >= rd) break;  // warp-uniform
+                    const uint32_t blk = e[q] >> 16;
+                    const bool high = e[q] >= kLowEnd;
+                    bool list = false;
+                    if (e[q] && !high) {
                         const int half = (int)(blk & 1u) * 16;
                         const uint32_t old = atomicOr(dir + (blk >> 1), (e[q] & 0xffffu) << half);
-                        nl += (int)(((old >> half) & 0xffffu) == 0);
-                        continue;
+                        const bool fresh = ((old >> half) & 0xffffu) == 0;
+                        nl += (int)fresh;
+                        list = fresh && blk >= (uint32_t)dn;
                     }
-                    uint32_t h = (blk * kHashMul) >> (32 - lg);
-                    for (int left = hn; left; --left) {  // at most half of the places are taken
-                        const uint32_t old = atomicCAS(hs + h, 0u, e[q]);
-                        if (old == 0u) {
-                            nl += (int)low;
-                            break;
-                        }
-                        if ((old < kLowEnd) == low && ((old ^ e[q]) >> sh) == 0) {
-                            atomicOr(hs + h, e[q]);
-                            break;
-                        }
-                        h = (h + 1u) & (uint32_t)(hn - 1);
+                    const uint32_t bh = __ballot_sync(kFull, high);
+                    if (high) out[o + __popc(bh & lt)] = e[q];
+                    o += __popc(bh);
+                    if (small) {
+                        const uint32_t b = __ballot_sync(kFull, list);
+                        if (list) s_list[warp][n_list + __popc(b & lt)] = (uint16_t)blk;
+                        n_list += __popc(b);
                     }
                 }
-                __syncwarp();
-                for (int w = lane; w < hn; w += kWarp) {  // hn is a multiple of 32
-                    const uint32_t v = hs[w];
-                    const bool high = v >= kLowEnd;
-                    const uint32_t b = __ballot_sync(kFull, high);
-                    if (high) {
-                        hs[w] = 0;
-                        out[o + __popc(b & lt)] = v;
-                    }
-                    o += __popc(b);
-                }
-                __syncwarp();
             }
+            __syncwarp();
             const int hq = (o + 3) >> 2;
             if (lane < 4 * hq - o) out[o + lane] = 0;
             // the low entries, ascending, eight blocks per lane at a time
@@ -467,16 +452,11 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
                 }
                 if (any) *d4 = make_uint4(0, 0, 0, 0);
             }
-            if (small) {
-                for (int w = lane; w < hn; w += kWarp) {  // what is left in the hash: low blocks
-                    const uint32_t v = hs[w];
-                    const uint32_t b = __ballot_sync(kFull, v != 0);
-                    if (v) {
-                        hs[w] = 0;
-                        lrow[deal(at + __popc(b & lt))] = v;
-                    }
-                    at += __popc(b);
-                }
+            for (int w = lane; w < n_list; w += kWarp) {
+                const int b = s_list[warp][w];
+                uint16_t *m = reinterpret_cast<uint16_t *>(dir) + b;
+                lrow[deal(at + w)] = ((uint32_t)b << 16) | *m;
+                *m = 0;
             }
             if (lane < 8 * deal.octets - nl) lrow[deal(nl + lane)] = 0;
             if (lane == k) *desc = make_int4((int)rq, hq, deal.octets, o + nl);
