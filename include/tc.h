@@ -100,8 +100,9 @@ TC_API int tc_ctx_device_info(tc_ctx *ctx, int *sm_count, size_t *free_bytes, si
  * back to linear probing for a task whose insertion gives up); 0 selects
  * linear probing.  (The default, a cuckoo table with neither heavy_bitmap,
  * hash_pairs nor intersect, counts skewed graphs on rows packed into blocks of
- * ids instead (csrc/tc_pack.cu; of these fields it uses warp_max_deg, unit_work
- * / 8192 out-neighbours per heavy unit, blocks_per_sm and flat_max_deg), and
+ * ids instead (csrc/tc_pack.cu; of these fields it uses warp_max_deg, twice it
+ * being the longest row of one warp, unit_work / 2048 out-neighbours per block
+ * unit, blocks_per_sm and flat_max_deg), and
  * with flat_max_deg > 0 graphs of few edges in one launch.)  heavy_bitmap = 1 runs heavy tasks on a direct-address
  * shared-memory bitmap of N+(x) (one load per probe) whenever the graphs'
  * vertex ids fit in one block's shared memory (about 1.85 M rows).

@@ -1,6 +1,6 @@
 """The packed-row count (tc_pack.cu) against the oracle and against the plain-id
 tables, at the sizes where its layout changes: row lengths around a window (32),
-a piece (128), the warp / block border (256) and a block's hash tile; ids around
+a piece (128), the warp / block border (512) and a block's hash tile; ids around
 the low blocks' end (30,720) and around the last full-width mask (63,488 x 16);
 graphs around the one-launch and the sampling bound; edges that follow no
 order."""
@@ -53,7 +53,8 @@ def check(ctx, rp, col, n_roots=None):
 
 
 @pytest.mark.parametrize("n", [4000, 40000])  # with and without high blocks
-@pytest.mark.parametrize("d", [1, 2, 3, 8, 9, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 1023, 1025, 3500])
+@pytest.mark.parametrize("d", [1, 2, 3, 8, 9, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513,
+                               1023, 1025, 3500])
 def test_row_lengths(chain, n, d):
     rp, col = rows_of_lengths([d, d, 32, d, 2, 33, d], n, d)
     check(chain, rp, col)

@@ -1155,8 +1155,12 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
         P.desc = ps.desc;
         P.mid_list = ps.mid_list;
         P.units = ps.units;
-        P.warp_max = std::min(tn.warp_max, 256);
-        P.slice = std::min(256, std::max(32, tn.unit_work / 8192));
+        // Rows of up to 512 (twice the tuning's bound) on one warp: a block's eight warps wait for one another around
+        // every unit's table (R-MAT 21 3.16 ms with 256, 3.00 with 512, 2.97 with no bound, whose last rows could be
+        // a warp's millisecond).  Units of 512 out-neighbours (unit_work / 2048): with 128 a row's table was built
+        // four times as often (3.37 ms; R-MAT 23's eight parts 32.9, 30.6 with 512).
+        P.warp_max = 2 * tn.warp_max;
+        P.slice = std::min(512, std::max(32, tn.unit_work / 2048));
         TC_CUDA(cudaMemsetAsync(ps.code, 0,
                                 sizeof(uint32_t) * ((size_t)total_vertices + (size_t)n_graphs * 2 * kBuckets), s));
         const int64_t tiles = (total_edges + kPopTile - 1) / kPopTile;
