@@ -592,35 +592,21 @@ int device_sm_count(int device) {
     return sm;
 }
 
+int longest_row(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int32_t *d_out) {
+    TC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(int32_t), ctx->stream));
+    if (n_rows > 0) max_row_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, d_out);
+    TC_CUDA(cudaGetLastError());
+    return TC_OK;
+}
+
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       tc_graph **out) {
+                       int32_t max_deg, tc_graph **out) {
     tc_graph *g = nullptr;
     TC_TRY(new_graph(ctx, n_rows, nnz, n_roots, &g));
     g->rp = rp;
     g->col = col;
     g->owns = true;
-    if (n_rows > 0) {  // the longest row, for the flat count
-        cudaStream_t s = ctx->stream;
-        DBuf<int> d;
-        int h = 0;
-        int st = d.alloc(1, s);
-        if (st == TC_OK && cudaMemsetAsync(d.p, 0, sizeof(int), s) != cudaSuccess) st = TC_E_CUDA;
-        if (st == TC_OK) {
-            max_row_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, d.p);
-            if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&h, d.p, sizeof(int), cudaMemcpyDeviceToHost, s) !=
-                                                         cudaSuccess ||
-                cudaStreamSynchronize(s) != cudaSuccess)
-                st = set_error(TC_E_CUDA, "row length scan failed");
-        }
-        if (st != TC_OK) {
-            g->owns = false;  // the caller still owns rp / col on failure
-            tc_graph_destroy(g);
-            return st;
-        }
-        g->max_deg = h;
-    } else {
-        g->max_deg = 0;
-    }
+    g->max_deg = max_deg;
     *out = g;
     return TC_OK;
 }

@@ -212,6 +212,9 @@ int scan_exclusive_i32_tmp(const int32_t *in, int32_t *out, int64_t n, int32_t *
 // is null.
 int scan_in_slots(unsigned long long *in_work, int32_t *in_off, int64_t n, int32_t *tmp, int64_t tmp_cap,
                   cudaStream_t s);
+// Local ids of a halo part's members: out[0..n] = exclusive scan of (part
+// vertices) + (halo vertices left) << 32 (cd: class, degree; out[n]: both totals).
+int scan_halo_ids(const int2 *cd, const uint8_t *removed, int64_t *out, int64_t n, cudaStream_t s);
 // LSD radix sort of n 64-bit keys on bits [0, bits).  Result in *keys (the
 // two buffers may be swapped).  tmp must hold n keys.
 int radix_sort_u64(uint64_t **keys, uint64_t **tmp, int64_t n, int bits, cudaStream_t s);

@@ -12,11 +12,12 @@
 // Halo extraction restates create_subgraph_with_halo
 // (preprocess_GPU/Halo_cleanned_preprocess/round_clean_subgraph.cu:357-902) with the
 // intended prune loop of Halo_creation_preprocess.py:566-589: the halo sets of
-// all parts from one pass (k <= 32); per part, local ids (part vertices, then
-// halo, each ascending) -> P/H/R class bits, tile counts and row-start ranks
-// over the orientation's tiles -> scan -> local row lengths and halo in-degrees
-// -> scan -> ordered write of every local edge; then halo vertices with zero
-// in-degree are peeled until none is left.
+// all parts from one pass (k <= 32); per part, P/H/R class bits, tile counts and
+// row-start ranks over the orientation's tiles -> scan -> row lengths and halo
+// in-degrees; halo vertices of zero in-degree are peeled on the undirected rows
+// until none is left; local ids (part vertices, then what is left of the halo,
+// each ascending) -> scan of the row lengths -> ordered write of every local
+// edge, once.
 #include <algorithm>
 #include <vector>
 
@@ -25,8 +26,10 @@
 namespace tc {
 
 int validate_csr(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_t n_rows, int64_t nnz);
+// Longest row (the out-degree bound that selects the flat count) into *d_out.
+int longest_row(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int32_t *d_out);
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       tc_graph **out);
+                       int32_t max_deg, tc_graph **out);
 
 namespace {
 
@@ -350,13 +353,11 @@ __global__ void __launch_bounds__(kOT) halo_mask_kernel(const int32_t *__restric
     if (m) atomicOr(mask + cur, m);
 }
 
-__global__ void part_halo_flags_kernel(const int32_t *part, const unsigned *mask, int64_t n, int p, uint8_t *inP,
-                                       uint8_t *inH) {
-    GRID_STRIDE(v, n) {
-        const bool in = part[v] == p;
-        inP[v] = (uint8_t)in;
-        inH[v] = (uint8_t)(!in && ((mask[v] >> p) & 1u));
-    }
+// cd[v] = (class, degree): 0 for a vertex of part p, 1 for one of its halo, -1
+// for the others; the tile pass gathers both with one load.
+__global__ void part_class_kernel(const int32_t *part, const unsigned *mask, const int32_t *deg, int64_t n, int p,
+                                  int2 *cd) {
+    GRID_STRIDE(v, n) cd[v] = make_int2(part[v] == p ? 0 : (int)((mask[v] >> p) & 1u) * 2 - 1, deg[v]);
 }
 
 // More than 32 parts: part p's flags, and its halo by one pass over the entries.
@@ -372,10 +373,8 @@ __global__ void halo_flags_kernel(const int32_t *rowid, const int32_t *col, int6
     }
 }
 
-// ld[v] = (local id or -1, degree): the tile passes gather both with one load.
-__global__ void local_ids_kernel(const uint8_t *inP, const uint8_t *inH, const int32_t *lidP, const int32_t *lidH,
-                                 const int32_t *deg, int64_t n, int t_ver, int2 *ld) {
-    GRID_STRIDE(v, n) ld[v] = make_int2(inP[v] ? lidP[v] : (inH[v] ? t_ver + lidH[v] : -1), deg[v]);
+__global__ void flag_class_kernel(const uint8_t *inP, const uint8_t *inH, const int32_t *deg, int64_t n, int2 *cd) {
+    GRID_STRIDE(v, n) cd[v] = make_int2(inP[v] ? 0 : (int)inH[v] * 2 - 1, deg[v]);
 }
 
 // Exclusive scan of one 64-bit value per thread over a 256-thread block.
@@ -407,15 +406,15 @@ __device__ __forceinline__ unsigned long long block_scan_256_u64(unsigned long l
 }
 
 // Local edges over the orientation's 4096-entry tiles.  Entry j (row s, id d)
-// is a local edge of the part when both ends have a local id and s -> d is the
-// oriented direction: a P entry when d is a part vertex (local id < t_ver),
-// else an H entry.  A local row lists its P entries, then its H entries, each
+// is a local edge of the part when both ends have a class and s -> d is the
+// oriented direction: a P entry when d is a part vertex (class 0), else an H
+// entry.  A local row lists its P entries, then its H entries, each
 // in the undirected row's (ascending) order, so an entry's offset in its local
 // row is its rank among the row's entries of its class (plus the row's P count
 // for an H entry).  Ranks come from the tiles' P and H counts, scanned, and one
 // block scan per tile, as in the orientation; no per-entry flag or position
 // array is written.  A third class, R, counts the halo in-degrees without
-// atomics: entry j of a halo row s is an R entry when d has a local id and
+// atomics: entry j of a halo row s is an R entry when d has a class and
 // d -> s is the oriented direction, so s's in-degree is its row's R count.
 //
 // Pass 1 (runs) stores the P and H bits of each thread's 16 entries (P in the
@@ -427,8 +426,8 @@ constexpr unsigned long long kRankMask = (1ull << kRankBits) - 1ull;
 
 __global__ void __launch_bounds__(kOT) halo_tile_count_kernel(const int32_t *__restrict__ rowid,
                                                                const int32_t *__restrict__ col,
-                                                               const int2 *__restrict__ ld, int64_t nnz, int64_t V,
-                                                               int64_t tiles, int t_ver, int tie,
+                                                               const int2 *__restrict__ cd, int64_t nnz, int64_t V,
+                                                               int64_t tiles, int tie,
                                                                uint32_t *__restrict__ bits,
                                                                int32_t *__restrict__ tile_cnt,
                                                                unsigned long long *__restrict__ row_rank) {
@@ -437,21 +436,21 @@ __global__ void __launch_bounds__(kOT) halo_tile_count_kernel(const int32_t *__r
     load16(rowid, col, j0, nnz, u, w);
     unsigned pb = 0, hb = 0, rb = 0;
     int cs = -1;
-    int2 cx = make_int2(-1, 0);  // the current row: local id, degree
+    int2 cx = make_int2(-1, 0);  // the current row: class, degree
 #pragma unroll
     for (int i = 0; i < kOI; ++i) {
         if (j0 + i >= nnz) break;
         if (u[i] != cs) {
             cs = u[i];
-            cx = __ldg(ld + cs);
+            cx = __ldg(cd + cs);
         }
         if (cx.x < 0) continue;
-        const int2 wx = __ldg(ld + w[i]);
+        const int2 wx = __ldg(cd + w[i]);
         if (wx.x < 0) continue;
         if (keep_edge(cx.y, wx.y, cs, w[i], tie)) {
-            if (wx.x < t_ver) pb |= 1u << i;
+            if (wx.x == 0) pb |= 1u << i;
             else hb |= 1u << i;
-        } else if (cx.x >= t_ver) {
+        } else if (cx.x == 1) {
             rb |= 1u << i;
         }
     }
@@ -491,27 +490,112 @@ __device__ __forceinline__ int halo_rank(int a, unsigned long long rk, const int
     return off[c * tiles + t] - off[c * tiles] + (int)((rk >> (c * kRankBits)) & kRankMask);
 }
 
+// Appends x to list, *n entries long, with one atomic for the lanes that are here
+// together (a frontier holds hundreds of thousands of vertices, and one atomic
+// each on the one counter was most of the peeling).
+__device__ __forceinline__ void push_together(int32_t *list, int32_t *n, int32_t x) {
+    const unsigned here = __activemask();
+    const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
+    int at = 0;
+    if (lane == first) at = atomicAdd(n, __popc(here));
+    at = __shfl_sync(here, at, first);
+    list[at + __popc(here & ((1u << lane) - 1u))] = x;
+}
+
 // Per vertex of the part's combined set: its P and H entry counts (from the
-// ranks at its row's start and at the next row's start) -> cnt[local id], the
-// bases that turn an entry's global rank into its local-row offset, and the
-// in-degree of a halo vertex (its row's R count; 0 for a part vertex).
-__global__ void halo_rows_kernel(const int32_t *__restrict__ rp, const int2 *__restrict__ ld,
+// ranks at its row's start and at the next row's start), the bases that turn an
+// entry's global rank into its local-row offset, and the in-degree of a halo
+// vertex (its row's R count).  Halo vertices of in-degree 0 are removed: they
+// make the first frontier.
+__global__ void halo_rows_kernel(const int32_t *__restrict__ rp, const int2 *__restrict__ cd,
                                  const unsigned long long *__restrict__ row_rank, const int32_t *__restrict__ off,
-                                 int64_t V, int64_t tiles, int t_ver, int32_t *__restrict__ cnt,
-                                 int32_t *__restrict__ base_p, int32_t *__restrict__ base_h,
-                                 int32_t *__restrict__ indeg) {
+                                 int64_t V, int64_t tiles, int32_t *__restrict__ cnt, int32_t *__restrict__ base_p,
+                                 int32_t *__restrict__ base_h, int32_t *__restrict__ indeg,
+                                 uint8_t *__restrict__ removed, int32_t *__restrict__ front, int32_t *front_n) {
     GRID_STRIDE(v, V) {
-        const int l = ld[v].x;
-        if (l < 0) continue;
+        const int c = cd[v].x;
+        if (c < 0) continue;
         const int a = rp[v], b = rp[v + 1];
         const unsigned long long ra = row_rank[v], rb = row_rank[v + 1];
         const int pa = halo_rank(a, ra, off, tiles, 0), np = halo_rank(b, rb, off, tiles, 0) - pa;
         const int ha = halo_rank(a, ra, off, tiles, 1), nh = halo_rank(b, rb, off, tiles, 1) - ha;
-        cnt[l] = np + nh;
+        cnt[v] = np + nh;
         base_p[v] = pa;       // P entry of rank x: local offset x - pa
         base_h[v] = ha - np;  // H entry of rank x: local offset np + (x - ha)
-        indeg[l] = l >= t_ver ? halo_rank(b, rb, off, tiles, 2) - halo_rank(a, ra, off, tiles, 2) : 0;
+        bool gone = false;
+        if (c == 1) {
+            const int in = halo_rank(b, rb, off, tiles, 2) - halo_rank(a, ra, off, tiles, 2);
+            indeg[v] = in;
+            gone = in == 0;
+        }
+        removed[v] = (uint8_t)gone;
+        if (gone) push_together(front, front_n, (int32_t)v);
     }
+}
+
+// Peel round r, eight lanes per frontier vertex (they are vertices of few
+// neighbours: none of lower degree is in the part or its halo): drop its
+// out-edges, read off its undirected row; halo targets reaching in-degree 0 join
+// the next frontier (exactly once: the 1 -> 0 transition).  It runs before any
+// local edge is written, so the edges are written once, without the removed
+// rows (an edge into a removed vertex comes from a removed one).  Frontier sizes
+// stay on the device so that several rounds go out per host check: fn[r % 3] is
+// round r's frontier size (front_a for even r, front_b for odd r), fn[(r + 1) %
+// 3] (zeroed by round r - 1, or before round 0) counts the next frontier, and
+// fn[(r + 2) % 3], which no block of round r reads, is zeroed for round r + 1.
+// A round whose frontier is empty does nothing.
+__global__ void peel_round_kernel(int32_t *front_a, int32_t *front_b, int32_t *fn, int r, const int32_t *rp,
+                                  const int32_t *col, const int2 *cd, int tie, int32_t *indeg, uint8_t *removed) {
+    const int32_t *front = (r & 1) ? front_b : front_a;
+    int32_t *next = (r & 1) ? front_a : front_b;
+    const int n_front = fn[r % 3];
+    int32_t *next_n = fn + (r + 1) % 3;
+    if (blockIdx.x == 0 && threadIdx.x == 0) fn[(r + 2) % 3] = 0;
+    const int l8 = threadIdx.x & 7;
+    const int64_t g0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 3;
+    for (int64_t f = g0; f < n_front; f += ng) {
+        const int x = front[f];
+        const int dx = cd[x].y;
+        const int j1 = rp[x + 1];
+        for (int j0 = rp[x] + l8; j0 < j1; j0 += 32) {  // four neighbours in flight per lane
+            int d[4];
+            int2 c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d[q] = j0 + 8 * q < j1 ? __ldg(col + j0 + 8 * q) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) c[q] = d[q] >= 0 ? __ldg(cd + d[q]) : make_int2(-1, 0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (c[q].x == 1 && keep_edge(dx, c[q].y, x, d[q], tie) && atomicSub(&indeg[d[q]], 1) == 1) {
+                    removed[d[q]] = 1;
+                    push_together(next, next_n, d[q]);
+                }
+        }
+    }
+}
+
+// Local ids (part vertices, then the halo that is left, each ascending) from the
+// scan of both (scan_halo_ids), -1 for the others; row lengths by local id; the
+// longest row.
+__global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__restrict__ removed,
+                                const int64_t *__restrict__ ids, const int32_t *__restrict__ cnt, int64_t V,
+                                int32_t *__restrict__ lid, int32_t *__restrict__ len, int32_t *longest) {
+    const int t_ver = (int)(ids[V] & 0xffffffffll);
+    int most = 0;
+    GRID_STRIDE(v, V) {
+        const int c = cd[v].x;
+        int l = -1;
+        if (c == 0) l = (int)(ids[v] & 0xffffffffll);
+        else if (c == 1 && !removed[v]) l = t_ver + (int)(ids[v] >> 32);
+        lid[v] = l;
+        if (l >= 0) {
+            len[l] = cnt[v];
+            most = max(most, cnt[v]);
+        }
+    }
+    most = __reduce_max_sync(kFull, most);
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(longest, most);
 }
 
 // Pass 2 (strided): ranks each tile's P and H entries again from the stored
@@ -520,7 +604,7 @@ __global__ void halo_rows_kernel(const int32_t *__restrict__ rp, const int2 *__r
 // consecutive positions.
 __global__ void __launch_bounds__(kOT) halo_tile_write_kernel(const int32_t *__restrict__ rowid,
                                                                const int32_t *__restrict__ col,
-                                                               const int2 *__restrict__ ld,
+                                                               const int32_t *__restrict__ lid,
                                                                const uint32_t *__restrict__ bits, int64_t nnz,
                                                                int64_t tiles, const int32_t *__restrict__ off,
                                                                const int32_t *__restrict__ lrp,
@@ -546,87 +630,16 @@ __global__ void __launch_bounds__(kOT) halo_tile_write_kernel(const int32_t *__r
         const bool kp = rw & 1u, kh = (rw >> 16) & 1u;
         const unsigned bp = __ballot_sync(kFull, kp), bh = __ballot_sync(kFull, kh);
         if (kp || kh) {
-            const int s = __ldg(rowid + j);
-            const int ls = __ldg(ld + s).x;
-            const int lr = __ldg(lrp + ls);
-            const int o = kp ? lr - __ldg(base_p + s) + pr + __popc(bp & lt) : lr - __ldg(base_h + s) + hr + __popc(bh & lt);
-            lcol[o] = __ldg(ld + __ldg(col + j)).x;
+            // (the target's and the row's loads side by side, before the row is asked about)
+            const int s = __ldg(rowid + j), to = __ldg(lid + __ldg(col + j));
+            const int base = kp ? __ldg(base_p + s) : __ldg(base_h + s);
+            const int ls = __ldg(lid + s);
+            const int lr = __ldg(lrp + max(ls, 0));
+            const int rank = kp ? pr + __popc(bp & lt) : hr + __popc(bh & lt);
+            if (ls >= 0) lcol[lr - base + rank] = to;  // else a removed row
         }
         pr += __popc(bp);
         hr += __popc(bh);
-    }
-}
-
-__global__ void frontier_init_kernel(const int32_t *indeg, int64_t n, int t_ver, uint8_t *removed, int32_t *front,
-                                     int32_t *front_n) {
-    GRID_STRIDE(i, n) {
-        if (i >= t_ver && indeg[i] == 0) {
-            removed[i] = 1;
-            front[atomicAdd(front_n, 1)] = (int32_t)i;
-        }
-    }
-}
-
-// Peel round r, one warp per frontier vertex: drop its out-edges; halo targets
-// reaching in-degree 0 join the next frontier (exactly once: the 1 -> 0
-// transition).  Frontier sizes stay on the device so that several rounds go
-// out per host check: fn[r % 3] is round r's frontier size (front_a for even r,
-// front_b for odd r), fn[(r + 1) % 3] (zeroed by round r - 1, or before round 0)
-// counts the next frontier, and fn[(r + 2) % 3], which no block of round r
-// reads, is zeroed for round r + 1.  fn[3] totals the frontier sizes.  A round
-// whose frontier is empty does nothing.
-__global__ void peel_round_kernel(int32_t *front_a, int32_t *front_b, int32_t *fn, int r, const int32_t *lrp,
-                                  const int32_t *lcol, int t_ver, int32_t *indeg, uint8_t *removed) {
-    const int32_t *front = (r & 1) ? front_b : front_a;
-    int32_t *next = (r & 1) ? front_a : front_b;
-    const int n_front = fn[r % 3];
-    int32_t *next_n = fn + (r + 1) % 3;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        fn[(r + 2) % 3] = 0;
-        fn[3] += n_front;
-    }
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t f = w0; f < n_front; f += nw) {
-        const int x = front[f];
-        for (int j = lrp[x] + lane; j < lrp[x + 1]; j += 32) {
-            const int d = lcol[j];
-            if (atomicSub(&indeg[d], 1) == 1 && d >= t_ver) {
-                removed[d] = 1;
-                next[atomicAdd(next_n, 1)] = d;
-            }
-        }
-    }
-}
-
-__global__ void alive_kernel(const uint8_t *removed, const int32_t *lrp, int64_t n, uint8_t *alive, int32_t *len) {
-    GRID_STRIDE(i, n) {
-        const bool a = !removed[i];
-        alive[i] = (uint8_t)a;
-        len[i] = a ? lrp[i + 1] - lrp[i] : 0;
-    }
-}
-
-__global__ void prune_rows_kernel(const uint8_t *alive, const int32_t *nid, const int32_t *newpos, int64_t n,
-                                  int32_t *rp2) {
-    GRID_STRIDE(i, n) {
-        if (alive[i]) rp2[nid[i]] = newpos[i];
-    }
-}
-
-// One warp per surviving local row: its entries, renumbered, at the row's new
-// start (consecutive lanes write consecutive positions).
-__global__ void prune_cols_kernel(const int32_t *__restrict__ lcol, const int32_t *__restrict__ lrp, int64_t n,
-                                  const uint8_t *__restrict__ alive, const int32_t *__restrict__ nid,
-                                  const int32_t *__restrict__ newpos, int32_t *__restrict__ col2) {
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = w0; i < n; i += nw) {
-        if (!alive[i]) continue;
-        const int a = lrp[i], b = lrp[i + 1], o = newpos[i] - a;
-        for (int e = a + lane; e < b; e += 32) col2[o + e] = nid[lcol[e]];
     }
 }
 
@@ -881,9 +894,13 @@ int tc_orient(tc_ctx *ctx, const tc_ugraph *ug, int tie, tc_graph **out) {
     } else {
         TC_CUDA(cudaMemsetAsync(orp.p, 0, sizeof(int32_t) * (size_t)(V + 1), s));
     }
-    TC_CUDA(cudaStreamSynchronize(s));
+    DBuf<int32_t> d_longest;
+    int32_t longest = 0;
+    TC_TRY(d_longest.alloc(1, s));
+    TC_TRY(longest_row(ctx, orp.p, V, d_longest.p));
+    TC_TRY(d2h_scalar(&longest, d_longest.p, s));
     tc_graph *g = nullptr;
-    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, &g));
+    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, longest, &g));
     orp.release();
     ocol.release();
     *out = g;
@@ -916,22 +933,27 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
     for (int64_t v = 0; v < V; ++v)
         if (part[v] < 0) return set_error(TC_E_RANGE, "part[%lld] = %d is negative", (long long)v, part[v]);
     const int64_t tiles = (nnz + kOTile - 1) / kOTile;
-    DBuf<int32_t> dpart, lidP, lidH, cnt, lrp, tile_cnt, tile_off, base_p, base_h;
-    DBuf<int2> ld;
+    const size_t nv = (size_t)std::max<int64_t>(V, 1);
+    DBuf<int32_t> dpart, lid, cnt, lrp, tile_cnt, tile_off, base_p, base_h, indeg, front, next, words;
+    DBuf<int64_t> ids;
+    DBuf<int2> cd;
     DBuf<uint32_t> bits, mask;
     DBuf<unsigned long long> row_rank;
-    DBuf<uint8_t> inP, inH;
-    TC_TRY(dpart.alloc((size_t)std::max<int64_t>(V, 1), s));
+    DBuf<uint8_t> inP, inH, removed;
+    TC_TRY(dpart.alloc(nv, s));
     if (V) TC_CUDA(cudaMemcpyAsync(dpart.p, part, sizeof(int32_t) * (size_t)V, cudaMemcpyHostToDevice, s));
-    TC_TRY(inP.alloc((size_t)V, s));
-    TC_TRY(inH.alloc((size_t)V, s));
-    TC_TRY(lidP.alloc((size_t)V + 1, s));
-    TC_TRY(lidH.alloc((size_t)V + 1, s));
-    TC_TRY(ld.alloc((size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(cnt.alloc((size_t)V + 1, s));
+    TC_TRY(lid.alloc(nv, s));
+    TC_TRY(ids.alloc((size_t)V + 1, s));
+    TC_TRY(cd.alloc(nv, s));
+    TC_TRY(cnt.alloc(nv, s));
     TC_TRY(lrp.alloc((size_t)V + 1, s));
-    TC_TRY(base_p.alloc((size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(base_h.alloc((size_t)std::max<int64_t>(V, 1), s));
+    TC_TRY(base_p.alloc(nv, s));
+    TC_TRY(base_h.alloc(nv, s));
+    TC_TRY(indeg.alloc(nv, s));
+    TC_TRY(removed.alloc(nv, s));
+    TC_TRY(front.alloc(nv, s));
+    TC_TRY(next.alloc(nv, s));
+    TC_TRY(words.alloc(4, s));  // three frontier sizes, the longest row
     TC_TRY(row_rank.alloc((size_t)V + 1, s));
     TC_TRY(bits.alloc((size_t)std::max<int64_t>(tiles, 1) * kOT, s));
     TC_TRY(tile_cnt.alloc((size_t)std::max<int64_t>(3 * tiles, 1), s));
@@ -946,122 +968,88 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
                                                               mask.p);
         TC_CUDA(cudaGetLastError());
     }
-    // one part; any failure returns its status (the caller frees all parts)
+    if (!masks) {
+        TC_TRY(inP.alloc(nv, s));
+        TC_TRY(inH.alloc(nv, s));
+    }
+    struct Back {  // what the host reads per part
+        int32_t words[4];
+        int64_t ids;
+        int32_t nnz;
+    } *back = (Back *)ctx->h_pinned;
+    // one part, with one look from the host (once its sizes are known); any
+    // failure returns its status (the caller frees all parts)
     auto one_part = [&](int p) -> int {
         if (masks) {
-            if (V) part_halo_flags_kernel<<<gV, 256, 0, s>>>(dpart.p, mask.p, V, p, inP.p, inH.p);
+            if (V) part_class_kernel<<<gV, 256, 0, s>>>(dpart.p, mask.p, ug->deg, V, p, cd.p);
         } else {
             if (V) part_flags_kernel<<<gV, 256, 0, s>>>(dpart.p, V, p, inP.p);
             TC_CUDA(cudaMemsetAsync(inH.p, 0, (size_t)V, s));
             if (nnz)
                 halo_flags_kernel<<<gE, 256, 0, s>>>(ug->rowid, ug->col, nnz, dpart.p, ug->deg, p, in_only, tie, inH.p);
+            if (V) flag_class_kernel<<<gV, 256, 0, s>>>(inP.p, inH.p, ug->deg, V, cd.p);
         }
         TC_CUDA(cudaGetLastError());
-        TC_TRY(scan_flags_u8(inP.p, lidP.p, V, s));
-        TC_TRY(scan_flags_u8(inH.p, lidH.p, V, s));
-        int32_t t_ver = 0, n_halo = 0;
-        TC_CUDA(cudaMemcpyAsync(&t_ver, lidP.p + V, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        TC_CUDA(cudaMemcpyAsync(&n_halo, lidH.p + V, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        TC_CUDA(cudaStreamSynchronize(s));
-        const int64_t n_comb = (int64_t)t_ver + n_halo;
-        if (V) local_ids_kernel<<<gV, 256, 0, s>>>(inP.p, inH.p, lidP.p, lidH.p, ug->deg, V, t_ver, ld.p);
-        DBuf<int32_t> indeg;
-        TC_TRY(indeg.alloc((size_t)std::max<int64_t>(n_comb, 1), s));
+        TC_CUDA(cudaMemsetAsync(words.p, 0, 4 * sizeof(int32_t), s));
         if (tiles) {
-            halo_tile_count_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, ld.p, nnz, V, tiles, t_ver, tie,
-                                                                    bits.p, tile_cnt.p, row_rank.p);
+            halo_tile_count_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, cd.p, nnz, V, tiles, tie, bits.p,
+                                                                    tile_cnt.p, row_rank.p);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(tile_cnt.p, tile_off.p, 3 * tiles, s));
             if (V)
-                halo_rows_kernel<<<gV, 256, 0, s>>>(ug->rp, ld.p, row_rank.p, tile_off.p, V, tiles, t_ver, cnt.p,
-                                                    base_p.p, base_h.p, indeg.p);
+                halo_rows_kernel<<<gV, 256, 0, s>>>(ug->rp, cd.p, row_rank.p, tile_off.p, V, tiles, cnt.p, base_p.p,
+                                                    base_h.p, indeg.p, removed.p, front.p, words.p);
             TC_CUDA(cudaGetLastError());
         } else {
-            TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * ((size_t)n_comb + 1), s));
-            TC_CUDA(cudaMemsetAsync(indeg.p, 0, sizeof(int32_t) * (size_t)std::max<int64_t>(n_comb, 1), s));
+            TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * nv, s));
+            TC_CUDA(cudaMemsetAsync(removed.p, 0, nv, s));
         }
-        TC_TRY(scan_exclusive_i32(cnt.p, lrp.p, n_comb, s));
-        int32_t lnnz = 0;
-        TC_TRY(d2h_scalar(&lnnz, lrp.p + n_comb, s));
-        DBuf<int32_t> lcol, front, next, fn;
-        DBuf<uint8_t> removed;
-        TC_TRY(lcol.alloc((size_t)lnnz, s));
+        // Peel halo vertices of zero in-degree until none is left: eight rounds,
+        // then four more per look while there is a frontier (each round that has
+        // one removes a vertex).  A counting halo has none: each of its vertices
+        // has an in-edge from the part.
+        int round = 0;
+        auto peel = [&](int n) {
+            for (; n > 0 && tiles && !in_only; --n, ++round)
+                peel_round_kernel<<<ctx->sm_count * 8, 256, 0, s>>>(front.p, next.p, words.p, round, ug->rp, ug->col,
+                                                                    cd.p, tie, indeg.p, removed.p);
+        };
+        peel(8);
+        TC_CUDA(cudaGetLastError());
+        for (;; peel(4)) {
+            TC_TRY(scan_halo_ids(cd.p, removed.p, ids.p, V, s));
+            TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
+            TC_CUDA(cudaMemsetAsync(words.p + 3, 0, sizeof(int32_t), s));
+            if (V) halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, words.p + 3);
+            TC_CUDA(cudaGetLastError());
+            TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
+            TC_CUDA(cudaMemcpyAsync(back->words, words.p, sizeof(back->words), cudaMemcpyDeviceToHost, s));
+            TC_CUDA(cudaMemcpyAsync(&back->ids, ids.p + V, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            TC_CUDA(cudaMemcpyAsync(&back->nnz, lrp.p + V, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+            TC_CUDA(cudaStreamSynchronize(s));
+            if (in_only || back->words[round % 3] == 0) break;
+        }
+        const int32_t t_ver = (int32_t)(back->ids & 0xffffffffll), n_halo = (int32_t)(back->ids >> 32);
+        const int32_t longest = back->words[3];
+        const int64_t n_local = (int64_t)t_ver + n_halo, lnnz = back->nnz;
+        DBuf<int32_t> rp, lcol;
+        TC_TRY(rp.alloc((size_t)n_local + 1, s));
+        TC_TRY(lcol.alloc((size_t)std::max<int64_t>(lnnz, 1), s));
+        TC_CUDA(cudaMemcpyAsync(rp.p, lrp.p, sizeof(int32_t) * ((size_t)n_local + 1), cudaMemcpyDeviceToDevice, s));
         if (tiles && lnnz)
-            halo_tile_write_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, ld.p, bits.p, nnz, tiles,
+            halo_tile_write_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, lid.p, bits.p, nnz, tiles,
                                                                     tile_off.p, lrp.p, base_p.p, base_h.p, lcol.p);
         TC_CUDA(cudaGetLastError());
-        // prune: peel halo vertices of zero in-degree until none is left
-        TC_TRY(removed.alloc((size_t)std::max<int64_t>(n_comb, 1), s));
-        TC_TRY(front.alloc((size_t)std::max<int32_t>(n_halo, 1), s));
-        TC_TRY(next.alloc((size_t)std::max<int32_t>(n_halo, 1), s));
-        TC_TRY(fn.alloc(4, s));
-        TC_CUDA(cudaMemsetAsync(removed.p, 0, (size_t)std::max<int64_t>(n_comb, 1), s));
-        TC_CUDA(cudaMemsetAsync(fn.p, 0, 4 * sizeof(int32_t), s));
-        if (n_comb) frontier_init_kernel<<<grid(n_comb, ctx), 256, 0, s>>>(indeg.p, n_comb, t_ver, removed.p, front.p, fn.p);
-        TC_CUDA(cudaGetLastError());
-        // kPeelBatch rounds per host check; each non-empty round removes at
-        // least one halo vertex, so at most n_halo of them are non-empty
-        constexpr int kPeelBatch = 4;
-        const int peel_grid = std::min(grid((int64_t)std::max<int32_t>(n_halo, 1) * 32, ctx), ctx->sm_count * 4);
-        int32_t hfn[4] = {0, 0, 0, 0};
-        int round = 0;
-        while (round <= n_halo) {
-            for (int q = 0; q < kPeelBatch; ++q, ++round)
-                peel_round_kernel<<<peel_grid, 256, 0, s>>>(front.p, next.p, fn.p, round, lrp.p, lcol.p, t_ver, indeg.p,
-                                                            removed.p);
-            TC_CUDA(cudaGetLastError());
-            TC_CUDA(cudaMemcpyAsync(hfn, fn.p, sizeof(hfn), cudaMemcpyDeviceToHost, s));
-            TC_CUDA(cudaStreamSynchronize(s));
-            if (hfn[round % 3] == 0) break;  // the next round's frontier is empty
-        }
-        const int64_t n_removed = (int64_t)hfn[3] + hfn[round % 3];
-        int32_t *out_rp = nullptr, *out_col = nullptr;
-        int64_t n_local = n_comb, out_nnz = lnnz;
-        if (n_removed == 0) {
-            DBuf<int32_t> rp_copy;
-            TC_TRY(rp_copy.alloc((size_t)n_comb + 1, s));
-            TC_CUDA(cudaMemcpyAsync(rp_copy.p, lrp.p, sizeof(int32_t) * ((size_t)n_comb + 1), cudaMemcpyDeviceToDevice, s));
-            out_rp = rp_copy.release();
-            out_col = lcol.release();
-        } else {
-            DBuf<uint8_t> alive;
-            DBuf<int32_t> len, nid, newpos, rp2, col2;
-            TC_TRY(alive.alloc((size_t)n_comb, s));
-            TC_TRY(len.alloc((size_t)n_comb, s));
-            TC_TRY(nid.alloc((size_t)n_comb + 1, s));
-            TC_TRY(newpos.alloc((size_t)n_comb + 1, s));
-            alive_kernel<<<grid(n_comb, ctx), 256, 0, s>>>(removed.p, lrp.p, n_comb, alive.p, len.p);
-            TC_CUDA(cudaGetLastError());
-            TC_TRY(scan_flags_u8(alive.p, nid.p, n_comb, s));
-            TC_TRY(scan_exclusive_i32(len.p, newpos.p, n_comb, s));
-            int32_t nl = 0, nn = 0;
-            TC_CUDA(cudaMemcpyAsync(&nl, nid.p + n_comb, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            TC_CUDA(cudaMemcpyAsync(&nn, newpos.p + n_comb, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            TC_CUDA(cudaStreamSynchronize(s));
-            n_local = nl;
-            out_nnz = nn;
-            TC_TRY(rp2.alloc((size_t)nl + 1, s));
-            TC_TRY(col2.alloc((size_t)std::max(nn, 1), s));
-            prune_rows_kernel<<<grid(n_comb, ctx), 256, 0, s>>>(alive.p, nid.p, newpos.p, n_comb, rp2.p);
-            TC_CUDA(cudaMemcpyAsync(rp2.p + nl, &nn, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-            if (lnnz)
-                prune_cols_kernel<<<grid(n_comb * 32, ctx), 256, 0, s>>>(lcol.p, lrp.p, n_comb, alive.p, nid.p,
-                                                                         newpos.p, col2.p);
-            TC_CUDA(cudaGetLastError());
-            TC_CUDA(cudaStreamSynchronize(s));
-            out_rp = rp2.release();
-            out_col = col2.release();
-        }
-        TC_CUDA(cudaStreamSynchronize(s));
-        const int ast = graph_adopt_device(ctx, out_rp, out_col, n_local, out_nnz, t_ver, &parts_out[p]);
-        if (ast != TC_OK) {
-            dfree(out_rp, s);
-            dfree(out_col, s);
+        const int ast = graph_adopt_device(ctx, rp.p, lcol.p, n_local, lnnz, t_ver, longest, &parts_out[p]);
+        if (ast == TC_OK) {
+            rp.release();
+            lcol.release();
         }
         return ast;
     };
     int st = TC_OK;
     for (int p = 0; p < k && st == TC_OK; ++p) st = one_part(p);
+    if (cudaStreamSynchronize(s) != cudaSuccess && st == TC_OK) st = set_error(TC_E_CUDA, "halo extraction failed");
     if (st != TC_OK)
         for (int p = 0; p < k; ++p) {
             tc_graph_destroy(parts_out[p]);

@@ -29,6 +29,18 @@ struct HighHalf {
     __device__ __forceinline__ int32_t operator[](int64_t i) const { return (int32_t)(p[i] >> 32); }
 };
 
+// Scan input: a halo part's members, part vertices (class 0) in the low half and
+// halo vertices (class 1) that are not removed in the high half.
+struct HaloMember {
+    const int2 *cd;
+    const uint8_t *removed;
+    __device__ __forceinline__ int64_t operator[](int64_t i) const {
+        const int c = cd[i].x;
+        const bool gone = removed[i] != 0;  // unset, and unused, for the others: loaded beside the class, not after it
+        return c == 0 ? 1 : (int64_t)(c == 1 && !gone) << 32;
+    }
+};
+
 template <class T>
 __device__ __forceinline__ T warp_incl_scan(T v, int lane) {
 #pragma unroll
@@ -285,6 +297,10 @@ int scan_in_slots(unsigned long long *in_work, int32_t *in_off, int64_t n, int32
     const HighHalf in{in_work};
     if (tmp) return scan_tmp_impl<HighHalf, int32_t>(in, in_off, n, tmp, tmp_cap, s, in_work);
     return scan_impl<HighHalf, int32_t>(in, in_off, n, s, in_work);
+}
+
+int scan_halo_ids(const int2 *cd, const uint8_t *removed, int64_t *out, int64_t n, cudaStream_t s) {
+    return scan_impl<HaloMember, int64_t>(HaloMember{cd, removed}, out, n, s);
 }
 
 int radix_sort_u64(uint64_t **keys, uint64_t **tmp, int64_t n, int bits, cudaStream_t s) {
