@@ -5,10 +5,10 @@
 //
 // Scan: reduce-then-scan over tiles of 4096 values (256 threads x 16, each
 // warp scanning runs of 32 consecutive values, so every access is
-// coalesced), the tile sums scanned recursively.  Radix sort: 8-bit digits, per pass
+// coalesced), the tile sums scanned recursively.  Radix sort: digits of up to 9 bits, per pass
 // (1) per-tile digit histograms, (2) one exclusive scan over the
 // digit-major histogram table, (3) a stable scatter in which each warp ranks
-// its contiguous 512-key segment with __match_any_sync and the block stages
+// its contiguous 256-key segment with __match_any_sync and the block stages
 // the tile in shared memory so that global writes are runs of equal digits.
 #include <algorithm>
 
@@ -171,85 +171,110 @@ int scan_impl(In in, Out *out, int64_t n, cudaStream_t s, unsigned long long *sl
 }
 
 // ---- radix sort ---------------------------------------------------------------------
-constexpr int kRadixBits = 8;
-constexpr int kBins = 1 << kRadixBits;
-constexpr int kWarps = kT / 32;
-constexpr int kSeg = kTile / kWarps;  // keys per warp segment (512)
+// 512 threads of eight keys per tile of 4096, digits of up to nine bits.  The
+// scatter is a chain of dependent steps per warp, so what bounds it is how many
+// warps are there to hide it: 256 threads of sixteen 64-bit keys held 115
+// registers, 16 warps per SM, and took 118 us per pass of 10 M keys (0.56
+// instructions per cycle); these hold 48 warps per SM, 78 us.  Nine bits
+// instead of eight save a pass where the keys' bits allow (36: four, not five).
+constexpr int kRT = 512;              // threads
+constexpr int kRItems = kTile / kRT;  // keys per thread
+constexpr int kMaxDigit = 9;
+constexpr int kBins = 1 << kMaxDigit;
+constexpr int kRWarps = kRT / 32;
+constexpr int kSeg = kTile / kRWarps;  // keys per warp segment (256)
+static_assert(kBins == kRT, "one thread per bin");
 
-__global__ void __launch_bounds__(kT) radix_hist_kernel(const uint64_t *keys, int64_t n, int shift, int n_tiles,
-                                                       int32_t *hist) {
+__global__ void __launch_bounds__(kRT) radix_hist_kernel(const uint64_t *keys, int64_t n, int shift, int digit,
+                                                        int n_tiles, int32_t *hist) {
     __shared__ int32_t h[kBins];
     h[threadIdx.x] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kTile;
-#pragma unroll 4
-    for (int k = 0; k < kItems; ++k) {
-        const int64_t i = base + (int64_t)k * kT + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & (kBins - 1)], 1);
+    const uint32_t mask = (1u << digit) - 1u;
+    uint32_t d[kRItems];
+#pragma unroll
+    for (int k = 0; k < kRItems; ++k) {
+        const int64_t i = base + (int64_t)k * kRT + threadIdx.x;
+        d[k] = i < n ? (uint32_t)(keys[i] >> shift) & mask : kBins;
     }
+#pragma unroll
+    for (int k = 0; k < kRItems; ++k)
+        if (d[k] < kBins) atomicAdd(&h[d[k]], 1);
     __syncthreads();
-    hist[(int64_t)threadIdx.x * n_tiles + blockIdx.x] = h[threadIdx.x];  // digit-major
+    if (threadIdx.x <= mask) hist[(int64_t)threadIdx.x * n_tiles + blockIdx.x] = h[threadIdx.x];  // digit-major
 }
 
-__global__ void __launch_bounds__(kT) radix_scatter_kernel(const uint64_t *keys, uint64_t *out, int64_t n, int shift,
-                                                          int n_tiles, const int32_t *offs) {
-    __shared__ int32_t wh[kWarps][kBins];  // per-warp digit counts -> warp offsets
-    __shared__ int32_t tile_start[kBins];   // digit start inside the tile
-    __shared__ int32_t glob[kBins];         // digit start in the output
+__global__ void __launch_bounds__(kRT, 3) radix_scatter_kernel(const uint64_t *keys, uint64_t *out, int64_t n,
+                                                              int shift, int digit, int n_tiles, const int32_t *offs) {
+    __shared__ uint16_t wh[kRWarps][kBins];  // per-warp digit counts -> offsets among the tile's keys
     __shared__ uint64_t stage[kTile];
+    int32_t *glob = reinterpret_cast<int32_t *>(&wh[0][0]);  // (once wh is done with) digit start in the output, less
+                                                             // its start inside the tile
+    int32_t *wsum = reinterpret_cast<int32_t *>(stage);      // (before the keys are staged)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kWarps * kBins; i += kT) (&wh[0][0])[i] = 0;
-    glob[threadIdx.x] = offs[(int64_t)threadIdx.x * n_tiles + blockIdx.x];
+    const uint32_t mask = (1u << digit) - 1u;
+    for (int i = threadIdx.x; i < kRWarps * kBins / 2; i += kRT) reinterpret_cast<uint32_t *>(&wh[0][0])[i] = 0;
+    const int32_t first = threadIdx.x <= mask ? offs[(int64_t)threadIdx.x * n_tiles + blockIdx.x] : 0;
     __syncthreads();
     const int64_t seg_base = (int64_t)blockIdx.x * kTile + (int64_t)w * kSeg;
-    uint64_t key[kItems];
-    int rank[kItems];
+    uint64_t key[kRItems];
+    int rank[kRItems];
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int r = 0; r < kItems; ++r) {
+    for (int r = 0; r < kRItems; ++r) {
         const int64_t i = seg_base + r * 32 + lane;
-        const bool valid = i < n;
-        key[r] = valid ? keys[i] : ~0ull;
-        const int d = valid ? (int)((key[r] >> shift) & (kBins - 1)) : kBins;  // kBins: padding
+        key[r] = i < n ? keys[i] : ~0ull;
+    }
+#pragma unroll
+    for (int r = 0; r < kRItems; ++r) {
+        const bool valid = seg_base + r * 32 + lane < n;
+        const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & mask : (uint32_t)kBins;  // kBins: padding
         const unsigned peers = __match_any_sync(kFull, d);
         int prior = 0;
         if (valid) prior = wh[w][d];
         __syncwarp();
         rank[r] = prior + __popc(peers & lt);
-        if (valid && (peers & lt) == 0) wh[w][d] = prior + __popc(peers);
+        if (valid && (peers & lt) == 0) wh[w][d] = (uint16_t)(prior + __popc(peers));
         __syncwarp();
     }
     __syncthreads();
-    // exclusive scan over warps for each digit, then over digits for the tile
-    {
+    int32_t my_glob;
+    {  // one digit per thread: exclusive over the warps, then over the digits
         const int d = threadIdx.x;
         int run = 0;
 #pragma unroll
-        for (int ww = 0; ww < kWarps; ++ww) {
+        for (int ww = 0; ww < kRWarps; ++ww) run += wh[ww][d];
+        const int incl = warp_incl_scan(run, lane);
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        int start = incl - run;
+        for (int ww = 0; ww < w; ++ww) start += wsum[ww];
+        my_glob = first - start;
+        int at = start;
+#pragma unroll
+        for (int ww = 0; ww < kRWarps; ++ww) {
             const int c = wh[ww][d];
-            wh[ww][d] = run;
-            run += c;
+            wh[ww][d] = (uint16_t)at;
+            at += c;
         }
-        int tot;
-        const int start = block_excl_scan<int>(run, &tot);
-        tile_start[d] = start;
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kItems; ++r) {
-        const int64_t i = seg_base + r * 32 + lane;
-        if (i < n) {
-            const int d = (int)((key[r] >> shift) & (kBins - 1));
-            stage[tile_start[d] + wh[w][d] + rank[r]] = key[r];
-        }
-    }
+    for (int r = 0; r < kRItems; ++r)
+        if (seg_base + r * 32 + lane < n) stage[wh[w][(uint32_t)(key[r] >> shift) & mask] + rank[r]] = key[r];
+    __syncthreads();
+    glob[threadIdx.x] = my_glob;
     __syncthreads();
     const int64_t rem = n - (int64_t)blockIdx.x * kTile;
     const int tile_n = rem < kTile ? (int)rem : kTile;
-    for (int i = threadIdx.x; i < tile_n; i += kT) {
-        const uint64_t k = stage[i];
-        const int d = (int)((k >> shift) & (kBins - 1));
-        out[glob[d] + (i - tile_start[d])] = k;
+#pragma unroll
+    for (int r = 0; r < kRItems; ++r) {
+        const int i = r * kRT + (int)threadIdx.x;
+        if (i < tile_n) {
+            const uint64_t k = stage[i];
+            out[glob[(uint32_t)(k >> shift) & mask] + i] = k;
+        }
     }
 }
 
@@ -306,15 +331,18 @@ int scan_halo_ids(const int2 *cd, const uint8_t *removed, int64_t *out, int64_t 
 int radix_sort_u64(uint64_t **keys, uint64_t **tmp, int64_t n, int bits, cudaStream_t s) {
     if (n <= 1 || bits <= 0) return TC_OK;
     const int64_t tiles64 = (n + kTile - 1) / kTile;
-    if (tiles64 * kBins >= INT32_MAX) return set_error(TC_E_RANGE, "radix sort of %lld keys is too large", (long long)n);
+    // digits of equal width, at most nine bits
+    const int passes = (bits + kMaxDigit - 1) / kMaxDigit, width = (bits + passes - 1) / passes;
+    if ((tiles64 << width) >= INT32_MAX) return set_error(TC_E_RANGE, "radix sort of %lld keys is too large", (long long)n);
     const int n_tiles = (int)tiles64;
     DBuf<int32_t> hist;
-    TC_TRY(hist.alloc((size_t)n_tiles * kBins + 1, s));
-    for (int shift = 0; shift < bits; shift += kRadixBits) {
-        radix_hist_kernel<<<n_tiles, kT, 0, s>>>(*keys, n, shift, n_tiles, hist.p);
+    TC_TRY(hist.alloc(((size_t)n_tiles << width) + 1, s));
+    for (int shift = 0; shift < bits; shift += width) {
+        const int digit = std::min(width, bits - shift);
+        radix_hist_kernel<<<n_tiles, kRT, 0, s>>>(*keys, n, shift, digit, n_tiles, hist.p);
         TC_CUDA(cudaGetLastError());
-        TC_TRY(scan_exclusive_i32(hist.p, hist.p, (int64_t)n_tiles * kBins, s));
-        radix_scatter_kernel<<<n_tiles, kT, 0, s>>>(*keys, *tmp, n, shift, n_tiles, hist.p);
+        TC_TRY(scan_exclusive_i32(hist.p, hist.p, (int64_t)n_tiles << digit, s));
+        radix_scatter_kernel<<<n_tiles, kRT, 0, s>>>(*keys, *tmp, n, shift, digit, n_tiles, hist.p);
         TC_CUDA(cudaGetLastError());
         std::swap(*keys, *tmp);
     }
