@@ -114,6 +114,7 @@ struct PackParams {
     int4 *desc;          // per vertex (pooled): (first quad, quads of high blocks, octets of low blocks, entries)
     uint32_t *mid_list;  // roots for one warp each, as global rows chunk * 32 + lane
     uint2 *units;        // block units: (global row, slice)
+    int zero_quad;       // a quad of ent past the rows', set to zeros
     int warp_max, slice;
     int rank_chunks;  // 32-row chunks per block of hist and assign
     int pack_rows;    // rows per warp of pack, and per grab of the short roots: a power of two, at most 32
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
     uint32_t *dir = s_dir[warp];
     for (int i = lane; i < kLow / 2; i += kWarp) dir[i] = 0;
     __syncwarp();
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.ent[(uint32_t)P.zero_quad] = make_uint4(0, 0, 0, 0);
     const uint32_t le = kFull >> (31 - lane), lt = le >> 1;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
     const int64_t nw = (int64_t)gridDim.x * kWarps;
@@ -475,7 +477,7 @@ struct Rows {
     const int32_t *__restrict__ col;
     const int4 *__restrict__ desc;
     const uint4 *__restrict__ ent;
-    int mb;
+    int mb, zero;  // zero: a quad of zeros
     __device__ __forceinline__ int4 row(int v) const {  // as desc; raw: the first member instead of the quad
         if (kRaw) {
             const int s = __ldg(rp + v), n = __ldg(rp + v + 1) - s;
@@ -496,6 +498,7 @@ struct Rows {
         }
         return __ldg(ent + ((uint32_t)first + (uint32_t)i));  // offsets wrap in 32 bits
     }
+    __device__ __forceinline__ uint4 at(int quad) const { return __ldg(ent + (uint32_t)quad); }
     __device__ __forceinline__ int bits() const { return kRaw ? 1 : mb; }
 };
 
@@ -507,6 +510,7 @@ __device__ __forceinline__ Rows<kRaw> rows_of(const PackParams &P, const GraphDe
     R.desc = P.desc + G.vbase;
     R.ent = P.ent;
     R.mb = G.mbits;
+    R.zero = P.zero_quad;
     return R;
 }
 
@@ -626,34 +630,32 @@ __device__ __forceinline__ uint32_t low_hits(const uint32_t *words, uint4 q) {
 
 // Up to 32 lists (one per lane: n steps, of one quad each from quad `first` on,
 // or of an octet's two, n quads apart; raw: of members below `end`) laid end to
-// end.  s_at, s_n: per warp and list that is not empty, its first quad less its
-// place, and (octets) its steps.
+// end.  ListAt, per warp and list that is not empty: its first quad less its
+// place, and the octets or the caller's word.
 template <bool kRaw>
-struct ListAt {
-    int off;
+struct alignas(8) ListAt {
+    int off, x;
 };
 template <>
-struct ListAt<true> {
-    int off, end;
+struct alignas(4) ListAt<true> {
+    int off, x, end;
 };
 struct ListSpan {
-    int excl, total;  // the lane's list's place; steps in all
+    int excl, total;  // the lane's list's place (out of reach when it has none); steps in all
     unsigned have;    // lanes with a list
-    bool mine;
 };
-template <bool kRaw, int kStep>
-__device__ __forceinline__ ListSpan span_lists(int n, int first, int end, int lane, ListAt<kRaw> *s_at,
-                                               uint16_t *s_n = nullptr, int *s_w = nullptr, int w = 0) {
+constexpr int kNoList = 0x7fffffff;
+template <bool kRaw>
+__device__ __forceinline__ ListSpan span_lists(int n, int first, int end, int x, int lane, ListAt<kRaw> *s_at) {
     ListSpan s;
     s.excl = warp_excl_scan(n, lane, &s.total);
-    s.mine = n > 0;
-    s.have = __ballot_sync(kFull, s.mine);
-    if (s.mine) {
-        const int i = __popc(s.have & ((1u << lane) - 1u));
-        s_at[i].off = first - (kRaw ? 4 : 1) * s.excl;
-        if constexpr (kRaw) s_at[i].end = end;
-        if constexpr (kStep == 2) s_n[i] = (uint16_t)n;
-        if (s_w) s_w[i] = w;
+    s.have = __ballot_sync(kFull, n > 0);
+    if (n > 0) {
+        ListAt<kRaw> a;
+        a.off = first - (kRaw ? 4 : 1) * s.excl;
+        a.x = x;
+        if constexpr (kRaw) a.end = end;
+        s_at[__popc(s.have & ((1u << lane) - 1u))] = a;
     }
     return s;
 }
@@ -666,32 +668,30 @@ __device__ __forceinline__ ListSpan span_lists(int n, int first, int end, int la
 template <bool kRaw, int kStep, bool kWord = false>
 struct ListWalk {
     const Rows<kRaw> &R;
-    const ListSpan &s;
     const ListAt<kRaw> *s_at;
-    const uint16_t *s_n;
-    const int *s_w;
-    int lane, k;
-    uint4 q[kStep];
-    int w;  // the lane's list's word
-    __device__ __forceinline__ ListWalk(const Rows<kRaw> &R, const ListSpan &s, int lane, const ListAt<kRaw> *s_at,
-                                        const uint16_t *s_n, const int *s_w = nullptr)
-        : R(R), s(s), s_at(s_at), s_n(s_n), s_w(s_w), lane(lane), k(-1), w(0) {}
-    __device__ __forceinline__ void load(int b, int b1) {
-        const unsigned o = (unsigned)(s.excl - b);
+    int lane, mark, k;  // mark: the lane's list's place, kNoList without one
+    __device__ __forceinline__ ListWalk(const Rows<kRaw> &R, const ListSpan &s, int lane, const ListAt<kRaw> *s_at)
+        : R(R), s_at(s_at), lane(lane), mark((s.have >> lane) & 1u ? s.excl : kNoList), k(-1) {}
+    __device__ __forceinline__ void load(int b, int b1, uint4 (&q)[kStep], int &w) {
+        const int o = mark - b;
         const uint32_t starts =
-            __reduce_or_sync(kFull, s.mine && s.excl < b1 && o < (unsigned)kWarp ? 1u << o : 0u);
+            __reduce_or_sync(kFull, (unsigned)o < (unsigned)min(kWarp, b1 - b) ? 1u << o : 0u);
         const int t = b + lane;
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) q[i] = make_uint4(0, 0, 0, 0);
-        const int at = max(0, k + __popc(starts & (kFull >> (31 - lane))));  // (a lane past b1 has the last list's)
-        const ListAt<kRaw> a = s_at[at];
-        int e = 0, n = 0;
-        if constexpr (kRaw) e = a.end;
-        if constexpr (kStep == 2) n = s_n[at];
-        if constexpr (kWord) w = s_w[at];
-        if (t < b1) {
-            q[0] = R.quad(a.off, t, e);
-            if constexpr (kStep == 2) q[1] = R.quad(a.off, t + n, 0);
+        const int at = k + __popc(starts & (kFull >> (31 - lane)));
+        if constexpr (kRaw) {
+            q[0] = make_uint4(0, 0, 0, 0);
+            if (t < b1) {
+                const ListAt<true> a = s_at[at];
+                if constexpr (kWord) w = a.x;
+                q[0] = R.quad(a.off, t, a.end);
+            }
+        } else {
+            // (a lane past b1 has the last list's place and loads the quad of zeros)
+            const ListAt<false> a = s_at[at];
+            if constexpr (kWord) w = a.x;
+            const bool in = t < b1;
+            q[0] = R.at(in ? a.off + t : R.zero);
+            if constexpr (kStep == 2) q[1] = R.at(in ? a.off + t + a.x : R.zero);
         }
         k += __popc(starts);
     }
@@ -699,28 +699,36 @@ struct ListWalk {
     // before this round's look-ups.
     template <class F>
     __device__ __forceinline__ void run(int b0, int b1, F f) {
-        if (b0 < b1) load(b0, b1);
-        for (int b = b0; b < b1; b += kWarp) {
-            uint4 c[kStep];
-#pragma unroll
-            for (int i = 0; i < kStep; ++i) c[i] = q[i];
-            const int cw = w;
-            if (b + kWarp < b1) load(b + kWarp, b1);
+        if (b0 >= b1) return;
+        uint4 p[kStep], q[kStep];
+        int pw = 0, qw = 0;
+        auto use = [&](uint4 (&c)[kStep], int w) {
 #pragma unroll
             for (int i = 0; i < kStep; ++i) {
-                if constexpr (kWord) f(c[i], cw);
+                if constexpr (kWord) f(c[i], w);
                 else f(c[i]);
             }
+        };
+        load(b0, b1, p, pw);
+        for (int b = b0;;) {
+            b += kWarp;
+            if (b < b1) load(b, b1, q, qw);
+            use(p, pw);
+            if (b >= b1) break;
+            b += kWarp;
+            if (b < b1) load(b, b1, p, pw);
+            use(q, qw);
+            if (b >= b1) break;
         }
     }
 };
 
 template <bool kRaw, int kStep, class F>
 __device__ __forceinline__ void flat_lists(const Rows<kRaw> &R, int first, int n, int end, int lane,
-                                           ListAt<kRaw> *s_at, uint16_t *s_n, F f) {
-    const ListSpan s = span_lists<kRaw, kStep>(n, first, end, lane, s_at, s_n);
+                                           ListAt<kRaw> *s_at, F f) {
+    const ListSpan s = span_lists<kRaw>(n, first, end, n, lane, s_at);
     __syncwarp();
-    ListWalk<kRaw, kStep> W(R, s, lane, s_at, s_n);
+    ListWalk<kRaw, kStep> W(R, s, lane, s_at);
     W.run(0, s.total, f);
     __syncwarp();  // s_at is rewritten by the next call
 }
@@ -730,16 +738,16 @@ __device__ __forceinline__ void flat_lists(const Rows<kRaw> &R, int first, int n
 // blocks' and the high blocks' quads apart.
 template <bool kRaw>
 __device__ __forceinline__ uint32_t stream_lists(const Rows<kRaw> &R, int p, const uint32_t *words, const uint32_t *hs, int lg, bool low,
-                                                 bool high, int lane, ListAt<kRaw> *s_at, uint16_t *s_n) {
+                                                 bool high, int lane, ListAt<kRaw> *s_at) {
     uint32_t hits = 0;
     const int mb = R.bits();
     int4 l = make_int4(0, 0, 0, 0);
     if (p >= 0) l = R.row(p);
     if (high)
-        flat_lists<kRaw, 1>(R, l.x, l.y, l.x + l.w, lane, s_at, s_n,
+        flat_lists<kRaw, 1>(R, l.x, l.y, l.x + l.w, lane, s_at,
                             [&](uint4 q) { hits += kRaw ? hash_hits(hs, lg + 1, mb, q) : filter_hits(hs, lg, mb, q); });
     if (!kRaw && low)
-        flat_lists<kRaw, 2>(R, l.x + l.y, l.z, 0, lane, s_at, s_n, [&](uint4 q) { hits += low_hits(words, q); });
+        flat_lists<kRaw, 2>(R, l.x + l.y, l.z, 0, lane, s_at, [&](uint4 q) { hits += low_hits(words, q); });
     return hits;
 }
 
@@ -747,7 +755,7 @@ __device__ __forceinline__ uint32_t stream_lists(const Rows<kRaw> &R, int p, con
 // hashes of at most kWarpTile of them at a time.
 template <bool kRaw>
 __device__ __forceinline__ uint32_t warp_row(const Rows<kRaw> &R, int x, int rs, int d, int lane, uint32_t *words,
-                                             uint32_t *hs, ListAt<kRaw> *s_at, uint16_t *s_n) {
+                                             uint32_t *hs, ListAt<kRaw> *s_at) {
     const int4 l = R.row(x);
     const int mb = R.bits();
     uint32_t hits = 0;
@@ -773,7 +781,7 @@ __device__ __forceinline__ uint32_t warp_row(const Rows<kRaw> &R, int x, int rs,
         __syncwarp();
         for (int j = 0; j < d; j += kWarp)
             hits += stream_lists<kRaw>(R, j + lane < d ? __ldg(R.col + rs + j + lane) : -1, words, hs, kLogWarpH - 1, t0 == 0,
-                                       t1 > t0, lane, s_at, s_n);
+                                       t1 > t0, lane, s_at);
         __syncwarp();
         t0 = t1;
     } while (t0 < l.y);
@@ -796,13 +804,12 @@ struct alignas(16) ShortState {
     int4 row[kRaw ? kWarp : kWarp / 2];
     int tab[kRaw ? kWarp : kWarp / 2];  // its hash: first place | log2 places << 16 | the root's number << 24
     int cnt[kRaw ? kWarp : kWarp / 2];  // its hits among the high blocks (per-root counts)
-    int word[kWarp];                    // per list: its root's tab
 };
 template <bool kRaw, bool kPerRoot>
 __device__ __forceinline__ uint32_t short_rows(const Rows<kRaw> &R, int64_t x, int rs, int d, int lane,
                                                uint32_t *words, uint32_t *hs, ShortState<kRaw> &S,
                                                ListAt<kRaw> *s_low,
-                                               ListAt<kRaw> *s_high, uint16_t *s_n, unsigned long long *per_root) {
+                                               ListAt<kRaw> *s_high, unsigned long long *per_root) {
     uint32_t acc = 0;
     const int mb = R.bits();
     const uint32_t le = kFull >> (31 - lane);
@@ -844,15 +851,15 @@ __device__ __forceinline__ uint32_t short_rows(const Rows<kRaw> &R, int64_t x, i
             if (lq == 0) pl.z = 0;  // nothing to find there
             if (hq == 0) pl.y = 0;
         }
-        const ListSpan lo = span_lists<kRaw, 2>(kRaw ? 0 : pl.z, low0, 0, lane, s_low, s_n);
-        const ListSpan hi = span_lists<kRaw, 1>(pl.y, pl.x, pl.x + pl.w, lane, s_high, nullptr, S.word, tab);
+        const ListSpan lo = span_lists<kRaw>(kRaw ? 0 : pl.z, low0, 0, pl.z, lane, s_low);
+        const ListSpan hi = span_lists<kRaw>(pl.y, pl.x, pl.x + pl.w, tab, lane, s_high);
         __syncwarp();
         if (hi.total > 0) {
             for (int i = lane; i < places; i += kWarp) hs[i] = 0;
             __syncwarp();
             each4(high, [&](uint32_t e) { hash_put(hs + (tab & 0xffff), (tab >> 16) & 31, mb, e); });
             __syncwarp();
-            ListWalk<kRaw, 1, true> H(R, hi, lane, s_high, s_n, S.word);
+            ListWalk<kRaw, 1, true> H(R, hi, lane, s_high);
             H.run(0, hi.total, [&](uint4 q, int w) {
                 const uint32_t hit = hash_hits(hs + (w & 0xffff), (w >> 16) & 31, mb, q);
                 acc += hit;
@@ -860,9 +867,15 @@ __device__ __forceinline__ uint32_t short_rows(const Rows<kRaw> &R, int64_t x, i
             });
             __syncwarp();
         }
-        // the next root's first round of loads goes out before the last look-ups of the root before
-        ListWalk<kRaw, 2> W(R, lo, lane, s_low, s_n);
-        if (!kRaw) W.load(0, starts & (starts - 1u) ? __shfl_sync(kFull, lo.excl, __ffs(starts & (starts - 1u)) - 1) : lo.total);
+        // The next root's first round of loads goes out before the last look-ups of the root before.
+        ListWalk<kRaw, kRaw ? 1 : 2> W(R, lo, lane, s_low);
+        uint4 q[kRaw ? 1 : 2];
+        int word = 0;
+        if constexpr (!kRaw) {
+            const uint32_t rest = starts & (starts - 1u);
+            const int end = rest ? __shfl_sync(kFull, lo.excl, __ffs(rest) - 1) : lo.total;
+            if (end > 0) W.load(0, end, q, word);
+        }
         int i_root = 0;
         for (uint32_t todo = kPerRoot || lo.total > 0 ? starts : 0u; todo; ++i_root) {
             const int a = __ffs(todo) - 1;  // the root's lanes [a, b), the next one's [b, b2)
@@ -870,26 +883,29 @@ __device__ __forceinline__ uint32_t short_rows(const Rows<kRaw> &R, int64_t x, i
             const int b = todo ? __ffs(todo) - 1 : wlen;
             const uint32_t todo2 = todo & (todo - 1u);
             const int b2 = todo2 ? __ffs(todo2) - 1 : wlen;
-            const int4 r = S.row[i_root];
             uint32_t hits = 0;
-            if (!kRaw) {
+            if constexpr (!kRaw) {
                 const int lo0 = __shfl_sync(kFull, lo.excl, a);
                 const int lo1 = b < kWarp ? __shfl_sync(kFull, lo.excl, b & 31) : lo.total;
                 const int lo2 = b2 < kWarp ? __shfl_sync(kFull, lo.excl, b2 & 31) : lo.total;
-                const bool own = lane >= a && lane < b && lo1 > lo0;
-                if (own) each4(mine, [&](uint32_t e) { low_put(words, e); });
-                __syncwarp();
-                for (int q0 = lo0; q0 < lo1; q0 += kWarp) {
-                    const uint4 c0 = W.q[0], c1 = W.q[1];
-                    if (q0 + kWarp < lo1) W.load(q0 + kWarp, lo1);
-                    else W.load(lo1, lo2);
-                    hits += low_hits(words, c0) + low_hits(words, c1);
+                if (lo1 > lo0) {
+                    const bool own = lane >= a && lane < b;
+                    if (own) each4(mine, [&](uint32_t e) { low_put(words, e); });
+                    __syncwarp();
+                    for (int q0 = lo0; q0 < lo1; q0 += kWarp) {
+                        const uint4 c0 = q[0], c1 = q[1];
+                        if (q0 + kWarp < lo1) W.load(q0 + kWarp, lo1, q, word);
+                        else if (lo2 > lo1) W.load(lo1, lo2, q, word);
+                        hits += low_hits(words, c0) + low_hits(words, c1);
+                    }
+                    __syncwarp();
+                    if (own) each4(mine, [&](uint32_t e) { low_put(words, e, false); });
+                    __syncwarp();  // the next root's entries go in
+                } else if (lo2 > lo1) {
+                    W.load(lo1, lo2, q, word);  // no round of this root did it
                 }
-                if (lo1 == lo0 && lo2 > lo1) W.load(lo1, lo2);  // no round of this root did it
-                __syncwarp();
-                if (own) each4(mine, [&](uint32_t e) { low_put(words, e, false); });
-                __syncwarp();  // the next root's entries go in
             }
+            const int4 r = S.row[i_root];
             if (kPerRoot) {
                 const unsigned s = __reduce_add_sync(kFull, hits);
                 const unsigned t = s + (unsigned)S.cnt[i_root];
@@ -930,13 +946,11 @@ template <bool kPerRoot>
 __global__ void __launch_bounds__(kThreads, kPackedMinBlocks) packed_kernel(PackParams P) {
     __shared__ __align__(16) uint32_t s_words[kWarps][kWarpWords];
     __shared__ ListAt<false> s_lists[kWarps][kWarp], s_high[kWarps][kWarp];
-    __shared__ uint16_t s_octets[kWarps][kWarp];
     __shared__ ShortState<false> s_short[kWarps];
     __shared__ unsigned s_unit;
     __shared__ int s_chunk;
     const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
     ListAt<false> *s_at = s_lists[warp];
-    uint16_t *s_n = s_octets[warp];
     unsigned long long acc = 0;  // this lane's hits for graph cur_g
     int cur_g = -1;
     auto flush = [&](int g) {
@@ -986,7 +1000,7 @@ __global__ void __launch_bounds__(kThreads, kPackedMinBlocks) packed_kernel(Pack
                     const int j = j0 + __shfl_sync(kFull, q, 0) * step;
                     if (j >= j1) break;
                     hits += stream_lists<false>(R, lane < step && j + lane < j1 ? __ldg(G.col + rs + j + lane) : -1,
-                                                words, hs, kLogBlockH - 1, t0 == 0, t1 > t0, lane, s_at, s_n);
+                                                words, hs, kLogBlockH - 1, t0 == 0, t1 > t0, lane, s_at);
                 }
                 __syncthreads();
                 t0 = t1;
@@ -1014,7 +1028,7 @@ __global__ void __launch_bounds__(kThreads, kPackedMinBlocks) packed_kernel(Pack
             const int x = (int)(row - (uint32_t)(G.chunk_base * kWarp));
             const int rs = __ldg(G.rp + x), d = __ldg(G.rp + x + 1) - rs;
             const uint32_t hits = warp_row<false>(rows_of<false>(P, G), x, rs, d, lane, s_words[warp],
-                                                  s_words[warp] + kLow / 2, s_at, s_n);
+                                                  s_words[warp] + kLow / 2, s_at);
             if (kPerRoot) {
                 const unsigned s = __reduce_add_sync(kFull, hits);
                 if (lane == 0) G.per_root[x] = s;
@@ -1051,7 +1065,7 @@ __global__ void __launch_bounds__(kThreads, kPackedMinBlocks) packed_kernel(Pack
             }
             if (d < 2 || d > kRowMax) d = 0;
             acc += short_rows<false, kPerRoot>(rows_of<false>(P, G), x, rs, d, lane, s_words[warp],
-                                               s_words[warp] + kLow / 2, s_short[warp], s_at, s_high[warp], s_n,
+                                               s_words[warp] + kLow / 2, s_short[warp], s_at, s_high[warp],
                                                G.per_root);
         }
     }
@@ -1074,6 +1088,7 @@ __global__ void __launch_bounds__(kThreads) single_kernel(GraphDesc G, int rows,
     R.desc = nullptr;
     R.ent = nullptr;
     R.mb = 1;
+    R.zero = 0;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
     const int64_t nw = (int64_t)gridDim.x * kWarps;
     unsigned long long acc = 0;
@@ -1085,12 +1100,12 @@ __global__ void __launch_bounds__(kThreads) single_kernel(GraphDesc G, int rows,
             d = __ldg(G.rp + x + 1) - rs;
         }
         acc += short_rows<true, kPerRoot>(R, x, rs, d > kRowMax ? 0 : d, lane, nullptr, s_hash[warp], s_short[warp], s_lists[warp],
-                                          s_high[warp], nullptr, G.per_root);
+                                          s_high[warp], G.per_root);
         for (unsigned todo = __ballot_sync(kFull, d > kRowMax); todo; todo &= todo - 1u) {
             const int k = __ffs(todo) - 1;
             const int rrs = __shfl_sync(kFull, rs, k), rd = __shfl_sync(kFull, d, k);
             const uint32_t hits = warp_row<true>(R, (int)(x0 + k), rrs, rd, lane, nullptr, s_hash[warp],
-                                                 s_lists[warp], nullptr);
+                                                 s_lists[warp]);
             acc += hits;
             if (kPerRoot) {
                 const unsigned s = __reduce_add_sync(kFull, hits);
@@ -1155,6 +1170,7 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
         P.desc = ps.desc;
         P.mid_list = ps.mid_list;
         P.units = ps.units;
+        P.zero_quad = (int)(uint32_t)((total_edges + kRowPad * total_vertices + 4) >> 2);  // see row_quad, pack_scratch_alloc
         // Rows of up to 512 (twice the tuning's bound) on one warp: a block's eight warps wait for one another around
         // every unit's table (R-MAT 21 3.16 ms with 256, 3.00 with 512, 2.97 with no bound, whose last rows could be
         // a warp's millisecond).  Units of 512 out-neighbours (unit_work / 2048): with 128 a row's table was built
