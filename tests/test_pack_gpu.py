@@ -83,7 +83,7 @@ def test_popular_far_members(chain):
 
 @pytest.mark.parametrize("m", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, (1 << 21) - 1, (1 << 21) + 4097])
 def test_edge_count_bounds(ctx, m):
-    """One launch up to 2^18 edges; a sample of the edges ranks the ids from 2^21 on."""
+    """One launch up to 2^18 edges; a sample of the edges ranks the ids from 2^18 on."""
     src, dst = gen.rmat(17 if m > 1 << 19 else 14, 24)
     rp, col, _ = oracle.pipeline(src, dst)
     col = col[:m]

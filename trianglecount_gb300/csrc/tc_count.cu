@@ -1548,7 +1548,7 @@ int resolve_tuning(const tc_tuning &t, int sm_count, Tuned *out) {
     if (occ < 1) return set_error(TC_E_INVALID, "count kernel does not fit on an SM with %zu B shared memory", r.smem);
     const int bps = t.blocks_per_sm > 0 ? std::min(t.blocks_per_sm, occ) : occ;
     r.blocks = sm_count * bps;
-    TC_TRY(pack_blocks(sm_count, t.blocks_per_sm, &r.pack_blocks));
+    TC_TRY(pack_blocks(sm_count, bps, occ, &r.pack_blocks));
     // The auxiliary kernels walk the 32-row chunks grid-stride.  With no more
     // blocks than fit on the GPU at once, the chunks in flight form one moving
     // window, so a batch touches its graphs (and their in-lists) one after the
@@ -1564,6 +1564,14 @@ int resolve_tuning(const tc_tuning &t, int sm_count, Tuned *out) {
     aux_occ = std::min(aux_occ, o);
     r.aux_blocks = sm_count * std::max(1, aux_occ);
     *out = r;
+    return TC_OK;
+}
+
+int zero_work(CountWork *work, unsigned long long *results, int n, cudaStream_t s) {
+    const size_t rb = sizeof(unsigned long long) * (size_t)n;
+    const bool joined = results == (unsigned long long *)(work + 1);  // one operation where they lie together
+    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork) + (joined ? rb : 0), s));
+    if (!joined) TC_CUDA(cudaMemsetAsync(results, 0, rb, s));
     return TC_OK;
 }
 
@@ -1622,8 +1630,7 @@ int launch_count(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, in
     // light tasks are listed as 32-bit global row indices
     if (total_chunks * kWarp >= ((int64_t)1 << 32))
         return set_error(TC_E_RANGE, "a count of more than 2^32 rows in one launch is not supported");
-    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork), s));
-    TC_CUDA(cudaMemsetAsync(results, 0, sizeof(unsigned long long) * (size_t)n_graphs, s));
+    TC_TRY(zero_work(work, results, n_graphs, s));
     int nl = 0;
     if (total_chunks > 0) {
         TC_CUDA(cudaMemsetAsync(sc.in_work, 0, sizeof(unsigned long long) * (size_t)total_vertices, s));
@@ -1672,8 +1679,7 @@ int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_
                 unsigned long long *result, unsigned long long *per_root, const Tuned &tn, cudaStream_t s,
                 int *launches, cudaEvent_t *kev) {
     if (max_deg > kMicroDeg) return set_error(TC_E_INVALID, "flat count needs rows of at most %d entries", kMicroDeg);
-    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork), s));
-    TC_CUDA(cudaMemsetAsync(result, 0, sizeof(unsigned long long), s));
+    TC_TRY(zero_work(work, result, 1, s));
     if (kev) TC_TRY(record_kernel_event(kev[0], s));
     if (n_roots > 0) {
         const int64_t want = (n_roots + kThreads - 1) / kThreads;
@@ -1727,8 +1733,7 @@ int launch_count_noalloc(const GraphDesc *d_desc, int64_t total_chunks, int64_t 
     P.count_blocks = tn.blocks;
     P.heavy_done = 0;
     P.intersect = 0;
-    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork), s));
-    TC_CUDA(cudaMemsetAsync(results, 0, sizeof(unsigned long long), s));
+    TC_TRY(zero_work(work, results, 1, s));
     if (total_chunks > 0) {
         TC_CUDA(cudaMemsetAsync(sc.in_work, 0, sizeof(unsigned long long) * (size_t)total_vertices, s));
         TC_CUDA(cudaMemsetAsync(sc.out_work, 0, sizeof(unsigned long long) * (size_t)total_vertices, s));

@@ -159,13 +159,17 @@ bool pack_fits(int64_t V, int64_t E);  // else the plain-id tables count it
 int pack_mask_bits(int64_t n_rows);
 int pack_scratch_alloc(PackScratch *ps, int64_t V, int64_t E, int n_graphs, cudaStream_t s);
 void pack_scratch_free(PackScratch *ps, cudaStream_t s);
-int pack_blocks(int sm_count, int blocks_per_sm, int *out);
+// The packed count's persistent grid, num / den of what fits (a grid kept below
+// occupancy leaves the same share of an SM free as the plain-id count's).
+int pack_blocks(int sm_count, int num, int den, int *out);
 int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, int64_t total_vertices,
                   int64_t total_edges, const PackScratch &ps, CountWork *work, unsigned long long *results,
                   bool per_root, const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev);
 // One-kernel count of a graph of few edges, on its own ids.
 int launch_single(const GraphDesc &d, CountWork *work, unsigned long long *result, const Tuned &tn, cudaStream_t s,
                   int *launches, cudaEvent_t *kev);
+// Zeroes a launch's work words and its n results.
+int zero_work(CountWork *work, unsigned long long *results, int n, cudaStream_t s);
 // Records a kernel-timing event on s; inside a stream capture (the plain
 // count's cached graph) as an external event node, so that every replay of
 // the captured chain records it too.

@@ -52,7 +52,7 @@ constexpr int kWarps = kThreads / kWarp;
 constexpr int kRowMax = 32;         // roots of at most this out-degree are counted several per warp
 constexpr int kBuckets = 256;       // popularity buckets
 constexpr int kPopTile = 4096;      // edges per block of pop
-constexpr int64_t kSampleEdges = 1 << 21;
+constexpr int64_t kSampleEdges = 1 << 18;  // (R-MAT 16 125 us with 2^21, where it is not sampled, 116 so)
 constexpr int kPopItems = kPopTile / kThreads;
 constexpr uint32_t kHashMul = 0x9E3779B1u;
 
@@ -1153,8 +1153,7 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
                   bool per_root, const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev) {
     if (total_chunks * kWarp >= ((int64_t)1 << 32))
         return set_error(TC_E_RANGE, "a count of more than 2^32 rows in one launch is not supported");
-    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork), s));
-    TC_CUDA(cudaMemsetAsync(results, 0, sizeof(unsigned long long) * (size_t)n_graphs, s));
+    TC_TRY(zero_work(work, results, n_graphs, s));
     int nl = 0;
     if (total_chunks > 0) {
         PackParams P;
@@ -1210,8 +1209,7 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
 
 int launch_single(const GraphDesc &d, CountWork *work, unsigned long long *result, const Tuned &tn, cudaStream_t s,
                   int *launches, cudaEvent_t *kev) {
-    TC_CUDA(cudaMemsetAsync(work, 0, sizeof(CountWork), s));
-    TC_CUDA(cudaMemsetAsync(result, 0, sizeof(unsigned long long), s));
+    TC_TRY(zero_work(work, result, 1, s));
     if (kev) TC_TRY(record_kernel_event(kev[0], s));
     if (d.n_roots > 0) {
         // few rows per warp while the warps do not fill the GPU
@@ -1229,11 +1227,11 @@ int launch_single(const GraphDesc &d, CountWork *work, unsigned long long *resul
     return TC_OK;
 }
 
-int pack_blocks(int sm_count, int blocks_per_sm, int *out) {
+int pack_blocks(int sm_count, int num, int den, int *out) {
     int occ = 0;
     TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, packed_kernel<false>, kThreads, 0));
     if (occ < 1) return set_error(TC_E_INVALID, "the packed count kernel does not fit on an SM");
-    *out = sm_count * (blocks_per_sm > 0 ? std::min(blocks_per_sm, occ) : occ);
+    *out = sm_count * std::max(1, occ * num / den);
     return TC_OK;
 }
 
