@@ -302,10 +302,12 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
     __syncwarp();
     if (blockIdx.x == 0 && threadIdx.x == 0) P.ent[(uint32_t)P.zero_quad] = make_uint4(0, 0, 0, 0);
     const uint32_t le = kFull >> (31 - lane), lt = le >> 1;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-    const int64_t nw = (int64_t)gridDim.x * kWarps;
-    const int per = kWarp / P.pack_rows;  // warps per 32-row chunk
-    for (int64_t i0 = w0; i0 < P.total_chunks * per; i0 += nw) {
+    const int per = kWarp / P.pack_rows;  // grabs per 32-row chunk
+    for (;;) {
+        unsigned grab = 0;
+        if (lane == 0) grab = atomicAdd(&P.work->aux_cursor[1], 1u);
+        const int64_t i0 = (int64_t)__shfl_sync(kFull, grab, 0);
+        if (i0 >= P.total_chunks * per) break;
         const int64_t c = i0 / per;
         const GraphDesc &G = P.gd[graph_of_chunk(P.gd, P.n_graphs, c)];
         const int32_t *__restrict__ col = G.col;
@@ -1194,7 +1196,7 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
         assign_kernel<<<rank_blocks, kThreads, 0, s>>>(P);
         TC_CUDA(cudaGetLastError());
         const int64_t want = (total_chunks * (kWarp / P.pack_rows) + kWarps - 1) / kWarps;
-        pack_kernel<<<(unsigned)std::min<int64_t>(want, (int64_t)tn.sm_count * 24), kThreads, 0, s>>>(P);
+        pack_kernel<<<(unsigned)std::min<int64_t>(want, (int64_t)tn.sm_count * 5), kThreads, 0, s>>>(P);
         TC_CUDA(cudaGetLastError());
         if (kev) TC_TRY(record_kernel_event(kev[0], s));
         if (per_root) packed_kernel<true><<<tn.pack_blocks, kThreads, 0, s>>>(P);
