@@ -329,7 +329,7 @@ class Context:
     def count(self, g: Graph, stats: bool = False):
         out = C.c_uint64()
         st = N.CountStats()
-        N.call("tc_count", self._h, g.handle, C.byref(out), C.byref(st))
+        N.call("tc_count", self._h, g.handle, C.byref(out), C.byref(st) if stats else None)
         if stats:
             return out.value, {"count_ms": st.count_ms, "finalize_ms": st.finalize_ms,
                                "launches": st.launches, "heavy_units": st.heavy_units}

@@ -336,7 +336,7 @@ int enqueue_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long
     unsigned long long *res = results ? results : g->d_result;
     if (flat_count(g)) {
         ctx->kev_recorded = true;
-        return launch_flat(g->rp, g->col, g->n_roots, g->max_deg, g->d_work, res, per_root, ctx->tuned, ctx->stream,
+        return launch_flat(g->rp, g->col, g->n_roots, g->max_deg, g->loop_free, g->d_work, res, per_root, ctx->tuned, ctx->stream,
                            launches, ctx->kev);
     }
     if (single_count(g)) {
@@ -607,6 +607,7 @@ int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, i
     g->col = col;
     g->owns = true;
     g->max_deg = max_deg;
+    g->loop_free = true;  // an undirected graph has no self-loop
     *out = g;
     return TC_OK;
 }
@@ -888,12 +889,12 @@ int tc_count(tc_ctx *ctx, tc_graph *g, uint64_t *out, tc_count_stats *stats) {
     cudaStream_t s = ctx->stream;
     int launches = 0;
     TC_TRY(prepare_graph_count(g, nullptr, nullptr));  // setup and any capture stay out of count_ms
-    TC_CUDA(cudaEventRecord(ctx->ev[0], s));
+    if (stats) TC_CUDA(cudaEventRecord(ctx->ev[0], s));
     TC_TRY(enqueue_graph_count(g, nullptr, nullptr, &launches));
-    TC_CUDA(cudaEventRecord(ctx->ev[1], s));
+    if (stats) TC_CUDA(cudaEventRecord(ctx->ev[1], s));
     TC_CUDA(cudaMemcpyAsync(ctx->h_pinned, g->d_work, sizeof(CountWork) + sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, s));
-    TC_CUDA(cudaEventRecord(ctx->ev[2], s));
+    if (stats) TC_CUDA(cudaEventRecord(ctx->ev[2], s));
     TC_CUDA(cudaStreamSynchronize(s));
     const CountWork *w = (const CountWork *)ctx->h_pinned;
     if (w->error) return set_error(TC_E_STATE, "%s", count_error_text(w->error));

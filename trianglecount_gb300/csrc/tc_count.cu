@@ -976,12 +976,15 @@ __global__ void __launch_bounds__(kThreads) flat_kernel(const int32_t *__restric
 // a root costs two dependent load rounds instead of four.  It runs one
 // resident wave (6 blocks per SM at 40 registers: the extra registers of the
 // pipeline spill at 32); road networks count ~30% faster than with a lane
-// per root.  The 8-wide count keeps the plain form: at 80 registers the
+// per root.  Roots of fewer than min_deg members have no hit (2 where no row
+// holds its own id): they load no neighbour, and two fifths of a road network's
+// roots have one member (1448 x 1448: 51 -> 46 us the call).  The 8-wide count keeps the plain form: at 80 registers the
 // pipelined one loses the residency it needs.
 template <bool kPerRoot>
 __global__ void __launch_bounds__(kThreads, kPerRoot ? 1 : 6) flat4_kernel(const int32_t *__restrict__ rp,
                                                                           const int32_t *__restrict__ col,
-                                                                          int64_t n_roots, unsigned long long *result,
+                                                                          int64_t n_roots, int min_deg,
+                                                                          unsigned long long *result,
                                                                           unsigned long long *per_root) {
     constexpr int D = 4;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1007,8 +1010,8 @@ __global__ void __launch_bounds__(kThreads, kPerRoot ? 1 : 6) flat4_kernel(const
         int ps[D], pe[D];
 #pragma unroll
         for (int i = 0; i < D; ++i) {
-            ps[i] = r[i] >= 0 ? __ldg(rp + r[i]) : 0;
-            pe[i] = r[i] >= 0 ? __ldg(rp + r[i] + 1) : 0;
+            ps[i] = r[i] >= 0 && d >= min_deg ? __ldg(rp + r[i]) : 0;
+            pe[i] = r[i] >= 0 && d >= min_deg ? __ldg(rp + r[i] + 1) : 0;
         }
         int rn[D];
 #pragma unroll
@@ -1675,7 +1678,7 @@ int launch_count(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, in
     return TC_OK;
 }
 
-int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_deg, CountWork *work,
+int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_deg, bool loop_free, CountWork *work,
                 unsigned long long *result, unsigned long long *per_root, const Tuned &tn, cudaStream_t s,
                 int *launches, cudaEvent_t *kev) {
     if (max_deg > kMicroDeg) return set_error(TC_E_INVALID, "flat count needs rows of at most %d entries", kMicroDeg);
@@ -1683,14 +1686,15 @@ int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_
     if (kev) TC_TRY(record_kernel_event(kev[0], s));
     if (n_roots > 0) {
         const int64_t want = (n_roots + kThreads - 1) / kThreads;
+        const int min_deg = loop_free ? 2 : 1;  // roots of fewer members have no hit
         if (max_deg <= 4) {  // one resident wave, several roots per lane
             int occ = 1;
             TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &occ, per_root ? flat4_kernel<true> : flat4_kernel<false>, kThreads, 0));
             const int blocks =
                 (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)tn.sm_count * std::max(occ, 1)));
-            if (per_root) flat4_kernel<true><<<blocks, kThreads, 0, s>>>(rp, col, n_roots, result, per_root);
-            else flat4_kernel<false><<<blocks, kThreads, 0, s>>>(rp, col, n_roots, result, per_root);
+            if (per_root) flat4_kernel<true><<<blocks, kThreads, 0, s>>>(rp, col, n_roots, min_deg, result, per_root);
+            else flat4_kernel<false><<<blocks, kThreads, 0, s>>>(rp, col, n_roots, min_deg, result, per_root);
         } else {
             const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)tn.blocks * 8));
             if (per_root) flat_kernel<true, kMicroDeg><<<blocks, kThreads, 0, s>>>(rp, col, n_roots, result, per_root);

@@ -182,9 +182,10 @@ int launch_count_noalloc(const GraphDesc *d_desc, int64_t total_chunks, int64_t 
                          unsigned long long *results, const Tuned &tn, cudaStream_t s);
 
 // One-kernel count of a graph whose rows are all at most max_deg <= 8 long
-// (one lane per root, lists in registers); fills the work words and result
+// (one lane per root, lists in registers; loop_free: no row holds its own id, so a
+// root with one member has no hit); fills the work words and result
 // like launch_count.
-int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_deg, CountWork *work,
+int launch_flat(const int32_t *rp, const int32_t *col, int64_t n_roots, int max_deg, bool loop_free, CountWork *work,
                 unsigned long long *result, unsigned long long *per_root, const Tuned &tn, cudaStream_t s,
                 int *launches, cudaEvent_t *kev);
 
@@ -269,6 +270,7 @@ struct tc_graph {
     int64_t n_rows = 0, nnz = 0, n_roots = 0;
     int32_t max_deg = -1;  // longest row, when known (uploads and device-built graphs)
     bool owns = true;
+    bool loop_free = false;  // no row holds its own id (device-built graphs)
     // per-graph count scratch, sized on first use
     tc::GraphDesc *d_desc = nullptr;
     tc::CountWork *d_work = nullptr;
