@@ -1196,7 +1196,8 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
         assign_kernel<<<rank_blocks, kThreads, 0, s>>>(P);
         TC_CUDA(cudaGetLastError());
         const int64_t want = (total_chunks * (kWarp / P.pack_rows) + kWarps - 1) / kWarps;
-        pack_kernel<<<(unsigned)std::min<int64_t>(want, (int64_t)tn.sm_count * 5), kThreads, 0, s>>>(P);
+        // five blocks fit an SM, or the share of them that the tuning leaves the packed grid
+        pack_kernel<<<(unsigned)std::min<int64_t>(want, (int64_t)tn.pack_blocks * 5 / kPackedMinBlocks), kThreads, 0, s>>>(P);
         TC_CUDA(cudaGetLastError());
         if (kev) TC_TRY(record_kernel_event(kev[0], s));
         if (per_root) packed_kernel<true><<<tn.pack_blocks, kThreads, 0, s>>>(P);
