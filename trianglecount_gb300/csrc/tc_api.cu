@@ -1164,11 +1164,14 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
     // average; the parts of one graph) are then counted on the context's
     // stream while the later parts are still being uploaded -- the copy
     // engine and the SMs work at the same time (R-MAT 23's eight parts: 3.3 GB
-    // of uploads in 16 ms under 41 ms of counts) -- in groups of 1, 2, 4, ...
+    // of uploads in 16 ms under 27 ms of counts) -- in groups of 1, 2, 3, ...
     // parts, one pooled launch per group (the last group takes the rest once
     // fewer than half the next group's size would be left): part 0 starts as
-    // soon as it is in, and the later groups pay one launch tail and one
-    // validation gap each instead of one per part.  Many small graphs are
+    // soon as it is in, the next group is about uploaded when the last one's
+    // count ends (a part counts in 1.5 x its upload), and a group pays one launch
+    // tail and one validation gap instead of one per part.  (Groups of 1, 2 and
+    // the other 5 waited for the whole upload: R-MAT 21's eight parts 7.0 instead
+    // of 6.2 ms.)  Many small graphs are
     // counted together in one batched launch once all are in (one launch each
     // would cost more than the copies).  The host waits only for verdicts.
     if (!ctx->aux[0]) {
@@ -1193,9 +1196,9 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
     }
     const bool overlap = n_parts <= 64 && sum_nnz / n_parts >= ((int64_t)1 << 22);
     std::vector<int> group_end;  // exclusive ends of the overlapped groups
-    for (int a = 0, sz = 1; overlap && a < n_parts; a = group_end.back(), sz *= 2) {
+    for (int a = 0, sz = 1; overlap && a < n_parts; a = group_end.back(), ++sz) {
         int b = std::min(n_parts, a + sz);
-        if (n_parts - b < sz) b = n_parts;
+        if (2 * (n_parts - b) < sz) b = n_parts;
         group_end.push_back(b);
     }
     std::vector<std::unique_ptr<PartGroup>> groups;
