@@ -22,9 +22,10 @@ Printed on rank 0 as ONE JSON line:
   e2e        the same metric through the C ABI (tc_count_parts_csr_i32) from
              pinned host buffers of the k = 8 parts: upload + validation +
              batched count + result read-back
-  roofline   of the dominant kernel (count_kernel of the batched launch):
-             achieved = the bytes this design must read (each root list, each
-             edge's row_ptr pair and the cheaper side's list) / its device time;
+  roofline   of the dominant kernel (packed_kernel of the batched launch):
+             achieved = the bytes of a count by cheaper sides on plain ids (each
+             root list, each edge's row_ptr pair and the cheaper side's list) / its
+             device time (the kernel itself reads packed entries of every list);
              the DRAM traffic of one launch (ncu) and the every-wedge byte
              model (every N+(v) read, the reference's probes) beside it
   cpu_baseline  the OpenMP merge-intersection oracle on the machine's host cores,
@@ -244,7 +245,7 @@ def run_reference(args, world, rank):
 
 
 def load_traffic(workload: str):
-    """DRAM traffic of one count_kernel launch from the committed ncu summary."""
+    """DRAM traffic of one counting kernel launch from the committed ncu summary."""
     p = os.path.join(ROOT, "profiles", f"count_kernel_{workload}.traffic.txt")
     if not os.path.exists(p):
         return None
@@ -405,13 +406,13 @@ def run_ours(args, world, rank, local, pg):
             "roofline": {"bound": "hbm", "achieved": B_min / sec / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": B_min / sec / 1e9 / peak, "peak_source": f"{peak_src} hbm_gbs (copy, burst)",
                          "kernel": (("flat4_kernel" if int(dplus.max(initial=0)) <= 4 else "flat_kernel") if flat
-                                    else "count_kernel"), "kernel_ms": kernel_avg_ms,
+                                    else "packed_kernel"), "kernel_ms": kernel_avg_ms,
                          "algorithmic_bytes_per_launch": B_min,
                          "algorithmic_bytes_definition": (
                              "4(V+1) + 12|E+| + 4 W+ + 8 (the flat kernel probes every wedge)" if flat else
                              "4(V+1) + 12|E+| + 4 sum_{u->v} min(d+(u), d+(v)) + 8: each root's row_ptr and list, "
-                             "each oriented edge's row_ptr pair and the cheaper side's list -- the bytes this "
-                             f"design must read ({P_min / max(W, 1):.2f} W+ probes on this graph)"),
+                             "each oriented edge's row_ptr pair and the cheaper side's list of plain ids "
+                             f"({P_min / max(W, 1):.2f} W+ on this graph; the packed count reads every list, packed)"),
                          "probes_done": probes,
                          "dram_achieved": traffic / sec / 1e9 if traffic else None,
                          "dram_frac": traffic / sec / 1e9 / peak if traffic else None,
@@ -419,8 +420,8 @@ def run_ours(args, world, rank, local, pg):
                          "traffic_source": (tr or {}).get("source"),
                          "wedge_model_bytes": B_alg, "wedge_model_frac": B_alg / sec / 1e9 / peak,
                          "wedge_model_note": "4(V+1) + 12|E+| + 4 W+ + 8 (every N+(v) read, W+ = sum over oriented "
-                                             "edges of d+(v)): work the min-side design does not do, so its "
-                                             "fraction can exceed 1 and is not evidence"},
+                                             "edges of d+(v)) as plain ids: the packed count reads fewer bytes, so "
+                                             "its fraction can exceed 1 and is not evidence"},
             "clocks": clk,
             "preprocess": {"clean_upload_s": round(clean_s, 4),
                            "clean_note": "host-timed: edge upload + device sort, dedupe, symmetrise, relabel",
@@ -746,18 +747,18 @@ def run_parts(args, world, rank, local, pg):
     sec = k_ms / 1000.0
     roofline = {"bound": "hbm", "achieved": B_min / sec / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": B_min / sec / 1e9 / peak, "traffic": traffic,
-                "peak_source": f"{peak_src} hbm_gbs (copy, burst)", "kernel": "count_kernel, the batched k = 8 count's two phase kernels (heavy units, then light tasks)",
+                "peak_source": f"{peak_src} hbm_gbs (copy, burst)", "kernel": "packed_kernel of the batched k = 8 count",
                 "kernel_ms": k_ms, "algorithmic_bytes_per_launch": B_min,
                 "algorithmic_bytes_definition": "sum over parts of 4(R+1) + 12 E_R + 4 sum_{u->v} min(d+(u), d+(v)) "
                                                 "+ 8 (R roots, E_R root edges): each root's row_ptr and list, each "
-                                                "root edge's row_ptr pair and the cheaper side's list -- the bytes "
-                                                "this design must read",
+                                                "root edge's row_ptr pair and the cheaper side's list of plain "
+                                                "ids (the packed count reads every list, packed)",
                 "dram_achieved": traffic / sec / 1e9 if traffic else None,
                 "dram_frac": traffic / sec / 1e9 / peak if traffic else None,
                 "traffic_source": (tr or {}).get("source"),
                 "wedge_model_bytes": B_model, "wedge_model_frac": B_model / sec / 1e9 / peak,
-                "wedge_model_note": "4(R+1) + 12 E_R + 4 W+ + 8 per part (every N+(v) read): work the min-side "
-                                     "design does not do, so its fraction can exceed 1 and is not evidence",
+                "wedge_model_note": "4(R+1) + 12 E_R + 4 W+ + 8 per part (every N+(v) read as plain ids): the packed "
+                                     "count reads fewer bytes, so its fraction can exceed 1 and is not evidence",
                 "W_plus": W_tot}
 
     # ---- end to end through the C ABI from pinned host memory (k = 8 parts) ----
@@ -944,7 +945,7 @@ def run_batch(args, world, rank, local, pg):
            "roofline": {"bound": "hbm", "achieved": B_min / (k_ms / 1000.0) / 1e9, "peak": peak, "unit": "GB/s",
                         "frac": B_min / (k_ms / 1000.0) / 1e9 / peak, "traffic": None,
                         "peak_source": f"{peak_src} hbm_gbs (copy, burst)",
-                        "kernel": "count_kernel (batched, 256 graphs)", "kernel_ms": k_ms,
+                        "kernel": "packed_kernel (batched, 256 graphs)", "kernel_ms": k_ms,
                         "algorithmic_bytes_per_launch": B_min,
                         "algorithmic_bytes_definition": "sum over graphs of 4(V+1) + 12|E+| + 4 sum_{u->v} "
                                                         "min(d+(u), d+(v)) + 8",
