@@ -791,7 +791,7 @@ def run_parts(args, world, rank, local, pg):
                     "ms_steps": [round(x, 2) for x in e2e_ms],
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 20 * len(pinned) + 48,
                     "path": "tc_count_parts_csr_i32: every part's upload issued at once; each part validated as "
-                            "soon as it is in; the parts counted in groups of 1, 2, then the rest, one launch per "
+                            "soon as it is in; the parts counted in groups of 1, 2, 3, ..., one launch per "
                             "group, under the later uploads; read-back"},
             "roofline": roofline, "clocks": clk, "detail": detail,
         }

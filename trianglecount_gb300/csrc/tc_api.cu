@@ -494,7 +494,8 @@ int graph_rebind(tc_graph *g, tc_ctx *ctx) {
 
 size_t graph_device_bytes(const tc_graph *g) {
     const size_t csr = sizeof(int32_t) * (size_t)(g->n_rows + 1 + g->nnz);
-    const size_t scratch = (size_t)(g->n_rows + 1) * (4 + 4 + 8 + 8 + 4 + 16) + (size_t)g->nnz * 5 + 1024;
+    // the larger of the two counts' scratch per row (packed: code, place, padding) and per edge
+    const size_t scratch = (size_t)(g->n_rows + 1) * (4 + 16 + 52) + (size_t)g->nnz * 5 + 4096;
     return csr + scratch;
 }
 

@@ -7,6 +7,11 @@
 // Every triangle u -> v -> w (u -> w) is found once, at its oriented edge u -> v
 // as the hit w of the intersection N+(u) n N+(v).
 //
+// Skewed graphs under the default tuning are counted on packed rows instead
+// (tc_pack.cu); this file has the count on plain ids, which serves the others,
+// the tunings that name a table form and the allocation-free count, and the
+// one-kernel count of bounded rows.
+//
 // The reference runs one 128-thread block per root and binary-searches each x
 // of N+(v) against 128-entry shared tiles of N+(u).  Here the intersection of
 // each oriented edge u -> v is done from its cheaper side:
