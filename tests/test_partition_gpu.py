@@ -121,3 +121,26 @@ def test_parts_equal_the_restatement(ctx, k, iterations):
     ug = ctx.upload_ugraph(rp, col)
     got = ctx.parts_lp(ug, k, seed=77, iterations=iterations)
     assert np.array_equal(got, lp_reference(rp, col, k, 77, iterations))
+
+
+@pytest.mark.parametrize("k", [8, 16])
+def test_half_a_million_vertices_every_time(ctx, k):
+    """n = 500 K against the restatement, from an edge list cleaned on the
+    device (the CSR is compared too, so that another graph and other parts are
+    told apart); then twenty calls per seed, other work on the context between
+    them, each on a CSR built anew."""
+    src, dst = gen.chung_lu(500_000, 16.0, seed=4)
+    rp, col = oracle.clean(src, dst)
+    ug = ctx.ugraph_from_edges(src, dst)
+    drp, dcol, _ = ug.download()
+    assert np.array_equal(drp, rp) and np.array_equal(dcol, col)
+    assert np.array_equal(ctx.parts_lp(ug, k, seed=77), lp_reference(rp, col, k, 77, 20))
+    busy = ctx.graph_from_edges(*gen.rmat(15))
+    for seed in range(10):
+        want = ctx.parts_lp(ug, k, seed=seed)
+        for i in range(20):
+            if i % 5 == 0:
+                again = ctx.ugraph_from_edges(src, dst)
+                ctx.count(busy)
+                ctx.count_per_root(busy)
+            assert np.array_equal(ctx.parts_lp(again, k, seed=seed), want)
