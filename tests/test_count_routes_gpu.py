@@ -1,0 +1,85 @@
+"""Which count a graph takes: the packed rows, the plain-id tables or one launch.
+The packed count is five launches; the plain-id count of more than 4096 rows at
+least seven (its scan alone takes three).  Every count is also checked against
+the oracle, on either side of each rule."""
+import numpy as np
+import pytest
+
+import oracle
+from trianglecount_gb300 import generators as gen
+
+pytestmark = pytest.mark.gpu
+
+PACKED = 5
+
+
+def csr(n, u, v):
+    key = np.unique(np.asarray(u, np.int64) * n + np.asarray(v, np.int64))
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(key // n, minlength=n), out=rp[1:])
+    return rp.astype(np.int32), (key % n).astype(np.int32)
+
+
+def by_rank(n, src, dst, rank):
+    """Every edge from its lower-ranked end to its higher-ranked one."""
+    keep = src != dst
+    s, d = src[keep], dst[keep]
+    swap = rank[s] > rank[d]
+    return csr(n, np.where(swap, d, s), np.where(swap, s, d))
+
+
+def by_degree(n, src, dst):
+    deg = np.bincount(np.concatenate((src, dst)), minlength=n).astype(np.int64)
+    return by_rank(n, src, dst, deg * n + np.arange(n))
+
+
+def with_clique(src, dst, size):
+    i, j = np.triu_indices(size, 1)
+    return np.concatenate((src, i + 5)), np.concatenate((dst, j + 5))
+
+
+def launches_of(ctx, rp, col, n_roots=None):
+    """Launches of one count; the count, the per-root counts and a batch against the oracle."""
+    want, pr = oracle.count(rp, col, n_roots=n_roots, per_root=True)
+    g = ctx.upload(rp, col, n_roots=n_roots)
+    got, st = ctx.count(g, stats=True)
+    assert got == want
+    assert np.array_equal(ctx.count_per_root(g), pr)
+    assert list(ctx.batch([g]).run()) == [want]
+    return st["launches"]
+
+
+def test_one_clique_does_not_make_a_graph_skewed(ctx):
+    """A few long rows in a graph without hubs: the plain-id tables, as without them."""
+    n = 100_000
+    src, dst = gen.er(n, 16.0, seed=3)
+    assert launches_of(ctx, *by_degree(n, src, dst)) > PACKED
+    src, dst = with_clique(src, dst, 90)
+    rp, col = by_degree(n, src, dst)
+    assert np.diff(rp).max() * n > 5 * len(col)
+    assert launches_of(ctx, rp, col) > PACKED
+    for tie in ("reference", "id_asc"):  # built on the device: whole, and as parts
+        g = ctx.graph_from_edges(src, dst, tie=tie)
+        assert ctx.count(g, stats=True)[1]["launches"] > PACKED
+    src, dst = gen.er(300_000, 16.0, seed=4)
+    ug = ctx.ugraph_from_edges(*with_clique(src, dst, 90))
+    part = gen.parts_random(ug.info()[0], 2)
+    for mode in ("reference", "count"):
+        for p in ctx.halo_extract(ug, part, 2, mode=mode):
+            assert p.n_rows > 61440 and ctx.count(p, stats=True)[1]["launches"] > PACKED
+
+
+@pytest.mark.parametrize("maker", ["rmat17", "rmat19", "chung_lu_8", "chung_lu_64"])
+def test_skewed_graphs_count_packed(ctx, maker):
+    src, dst = {"rmat17": lambda: gen.rmat(17), "rmat19": lambda: gen.rmat(19),
+                "chung_lu_8": lambda: gen.chung_lu(80_000, 8.0, seed=1),
+                "chung_lu_64": lambda: gen.chung_lu(80_000, 64.0, seed=1)}[maker]()
+    g = ctx.graph_from_edges(src, dst)
+    rp, col = g.download()
+    assert g.n_rows > 61440
+    assert ctx.count(g, stats=True)[1]["launches"] == PACKED
+    assert launches_of(ctx, rp, col) == PACKED
+    ug = ctx.ugraph_from_edges(src, dst)
+    parts = ctx.halo_extract(ug, gen.parts_random(ug.info()[0], 3), 3, mode="count")
+    assert [ctx.count(p, stats=True)[1]["launches"] for p in parts] == [PACKED] * 3
+    assert sum(ctx.count(p) for p in parts) == oracle.count(rp, col)

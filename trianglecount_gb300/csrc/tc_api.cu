@@ -23,14 +23,16 @@ constexpr int32_t kSingleMaxDeg = 64;
 
 // ---- CSR validation (rows strictly ascending, ids in range) ----
 struct ValidateErr {
-    int code;     // 0 ok, 1 row_ptr, 2 id range, 3 order
-    int first;    // smallest offending row / entry index
-    int max_deg;  // longest row
+    int code;       // 0 ok, 1 row_ptr, 2 id range, 3 order
+    int first;      // smallest offending row / entry index
+    RowStats rows;  // of valid rows
 };
+constexpr ValidateErr kNoErr{0, 0x7fffffff, {0, 0}};
 
-__global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz, uint8_t *start, ValidateErr *err) {
+__global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz, int skew, uint8_t *start,
+                                 ValidateErr *err) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int longest = 0;
+    RowTally t;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n_rows; u += stride) {
         const int64_t a = rp[u], b = rp[u + 1];
         const bool bad = a > b || a < 0 || b > nnz || (u == 0 && a != 0) || (u == n_rows - 1 && b != nnz);
@@ -39,21 +41,18 @@ __global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz,
             atomicMin(&err->first, (int)u);
         } else if (a < b) {
             start[a] = 1;
-            longest = max(longest, (int)(b - a));
+            t.row((int)(b - a), skew);
         }
     }
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    if ((threadIdx.x & 31) == 0 && longest) atomicMax(&err->max_deg, longest);
+    t.add(&err->rows);
 }
 
-// Longest row of a CSR (the out-degree bound that selects the flat count).
-__global__ void max_row_kernel(const int32_t *rp, int64_t n_rows, int *out) {
+__global__ void row_stats_kernel(const int32_t *rp, int64_t n_rows, int skew, RowStats *out) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int longest = 0;
+    RowTally t;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n_rows; u += stride)
-        longest = max(longest, rp[u + 1] - rp[u]);
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    if ((threadIdx.x & 31) == 0 && longest) atomicMax(out, longest);
+        t.row(rp[u + 1] - rp[u], skew);
+    t.add(out);
 }
 
 // Four entries per thread: one 16-byte load of col[j..j+4), the next entry
@@ -103,17 +102,18 @@ int grid_for(int64_t n, int sm) {
 }
 
 int validate_csr_impl(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_t n_rows, int64_t nnz,
-                      int32_t *max_deg = nullptr) {
+                      RowStats *rows = nullptr) {
     cudaStream_t s = ctx->stream;
     DBuf<uint8_t> start;
     DBuf<ValidateErr> err;
     TC_TRY(start.alloc((size_t)nnz + 1, s));
     TC_TRY(err.alloc(1, s));
     TC_CUDA(cudaMemsetAsync(start.p, 0, (size_t)nnz + 1, s));
-    ValidateErr init{0, 0x7fffffff, 0};
+    const ValidateErr init = kNoErr;
     TC_CUDA(cudaMemcpyAsync(err.p, &init, sizeof(init), cudaMemcpyHostToDevice, s));
     if (n_rows > 0) {
-        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, start.p, err.p);
+        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, skew_bound(n_rows, nnz), start.p,
+                                                                         err.p);
         TC_CUDA(cudaGetLastError());
     }
     if (nnz > 0) {
@@ -129,7 +129,7 @@ int validate_csr_impl(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_
     case 2: return set_error(TC_E_FORMAT, "column id out of range [0, %lld) at entry %d", (long long)n_rows, h.first);
     case 3: return set_error(TC_E_FORMAT, "row not strictly ascending at entry %d", h.first);
     default:
-        if (max_deg) *max_deg = h.max_deg;
+        if (rows) *rows = h.rows;
         return TC_OK;
     }
 }
@@ -139,12 +139,12 @@ int validate_csr_impl(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_
 int validate_csr_enqueue(tc_ctx *ctx, cudaStream_t s, const int32_t *rp, const int32_t *col, int64_t n_rows,
                          int64_t nnz, uint8_t *start, ValidateErr *d_err) {
     TC_CUDA(cudaMemsetAsync(start, 0, (size_t)nnz + 1, s));
-    const ValidateErr init{0, 0x7fffffff, 0};
     // a parameter of a one-thread kernel, not a copy from this stack frame
-    set_validate_err_kernel<<<1, 1, 0, s>>>(d_err, init);
+    set_validate_err_kernel<<<1, 1, 0, s>>>(d_err, kNoErr);
     TC_CUDA(cudaGetLastError());
     if (n_rows > 0) {
-        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, start, d_err);
+        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, skew_bound(n_rows, nnz), start,
+                                                                         d_err);
         TC_CUDA(cudaGetLastError());
     }
     if (nnz > 0) {
@@ -154,15 +154,15 @@ int validate_csr_enqueue(tc_ctx *ctx, cudaStream_t s, const int32_t *rp, const i
     return TC_OK;
 }
 
-// The verdict of validate_csr_enqueue as a status (max_deg: the longest row).
-int validate_verdict(const ValidateErr &h, int64_t n_rows, int64_t nnz, int32_t *max_deg) {
+// The verdict of validate_csr_enqueue as a status.
+int validate_verdict(const ValidateErr &h, int64_t n_rows, int64_t nnz, RowStats *rows) {
     if (n_rows == 0 && nnz != 0) return set_error(TC_E_FORMAT, "CSR has 0 rows but %lld entries", (long long)nnz);
     switch (h.code) {
     case 1: return set_error(TC_E_FORMAT, "row_ptr is not a valid offset array at row %d", h.first);
     case 2: return set_error(TC_E_FORMAT, "column id out of range [0, %lld) at entry %d", (long long)n_rows, h.first);
     case 3: return set_error(TC_E_FORMAT, "row not strictly ascending at entry %d", h.first);
     default:
-        if (max_deg) *max_deg = h.max_deg;
+        if (rows) *rows = h.rows;
         return TC_OK;
     }
 }
@@ -247,22 +247,27 @@ void capture_count(tc_graph *g, unsigned long long *res) {
     cudaGetLastError();  // a failed capture falls back to direct launches
 }
 
-bool flat_count(const tc_graph *g) { return g->max_deg >= 0 && g->max_deg <= g->ctx->tuned.flat_max_deg; }
+bool flat_count(const tc_graph *g) {
+    return g->rows.longest >= 0 && g->rows.longest <= g->ctx->tuned.flat_max_deg;
+}
 
-// The packed count serves launches whose graphs are skewed (their longest row,
-// where it is known, above kSkew x the mean) or small enough that most ids are
-// low blocks'.  Without hubs the entries hold one id each and lie in the high
-// blocks, whose hashes cost more than the plain-id tables: Erdos-Renyi n = 1 M of
-// mean degree 8 / 40, longest rows 3.3 / 2.4 x the mean, 0.25 / 1.37 ms there,
-// 0.37 / 1.6 packed; n = 30 K of mean degree 40 0.18 and 0.16.  (R-MAT and
-// Chung-Lu graphs of the same sizes have 6 to 60 x the mean.)
-constexpr int64_t kSkew = 5, kPackRows = 61440;
+// The packed count serves launches whose graphs are skewed (at least 1 / kSkewShare
+// of their entries in rows longer than kSkew x the mean, where the rows are
+// known) or small enough that most ids are low blocks'.  Without hubs the entries
+// hold one id each and lie in the high blocks, whose hashes cost more than the
+// plain-id tables: Erdos-Renyi n = 1 M of mean degree 8 / 40 0.25 / 1.36 ms there,
+// 0.32 / 1.9 packed; n = 30 K of mean degree 40 0.18 and 0.16.  Degree-oriented
+// R-MAT graphs have 0.36 to 0.58 of their entries in such rows, Chung-Lu graphs
+// 0.08 to 0.26; an Erdos-Renyi graph of 8 M edges with a tenth of its edges in
+// cliques of 60 has 0.06 (0.67 ms plain, 0.76 packed).  One long row says nothing.
+constexpr int64_t kSkewShare = 16, kPackRows = 61440;
+bool skewed(const tc_graph *g) { return g->rows.longest < 0 || kSkewShare * g->rows.skewed >= g->nnz; }
 bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     if (!packed_count(tn)) return false;
     int64_t V = 0, E = 0, gain = 0;
     for (int i = 0; i < n; ++i) {
         const tc_graph *g = gs[i];
-        if (g->max_deg < 0 || g->n_rows <= kPackRows || g->max_deg * g->n_rows > kSkew * g->nnz) gain += g->nnz;
+        if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
         V += g->n_rows + 1;
         E += g->nnz;
     }
@@ -275,7 +280,7 @@ bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned
 bool single_count(const tc_graph *g) {
     const Tuned &tn = g->ctx->tuned;
     return packed_count(tn) && tn.flat_max_deg > 0 && !flat_count(g) && g->n_rows >= kSingleMinRows &&
-           g->nnz <= (g->max_deg >= 0 && g->max_deg <= kSingleMaxDeg ? kSingleMaxEdges : kSingleMaxSkewed);
+           g->nnz <= (g->rows.longest >= 0 && g->rows.longest <= kSingleMaxDeg ? kSingleMaxEdges : kSingleMaxSkewed);
 }
 
 // Everything a count of g needs before its launches: the work words, the
@@ -336,8 +341,8 @@ int enqueue_graph_count(tc_graph *g, unsigned long long *per_root, unsigned long
     unsigned long long *res = results ? results : g->d_result;
     if (flat_count(g)) {
         ctx->kev_recorded = true;
-        return launch_flat(g->rp, g->col, g->n_roots, g->max_deg, g->loop_free, g->d_work, res, per_root, ctx->tuned, ctx->stream,
-                           launches, ctx->kev);
+        return launch_flat(g->rp, g->col, g->n_roots, g->rows.longest, g->loop_free, g->d_work, res, per_root, ctx->tuned,
+                           ctx->stream, launches, ctx->kev);
     }
     if (single_count(g)) {
         ctx->kev_recorded = true;
@@ -593,21 +598,23 @@ int device_sm_count(int device) {
     return sm;
 }
 
-int longest_row(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int32_t *d_out) {
-    TC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(int32_t), ctx->stream));
-    if (n_rows > 0) max_row_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, d_out);
+int row_stats(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int64_t nnz, RowStats *d_out) {
+    TC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(RowStats), ctx->stream));
+    if (n_rows > 0)
+        row_stats_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, skew_bound(n_rows, nnz),
+                                                                                   d_out);
     TC_CUDA(cudaGetLastError());
     return TC_OK;
 }
 
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       int32_t max_deg, tc_graph **out) {
+                       const RowStats &rows, tc_graph **out) {
     tc_graph *g = nullptr;
     TC_TRY(new_graph(ctx, n_rows, nnz, n_roots, &g));
     g->rp = rp;
     g->col = col;
     g->owns = true;
-    g->max_deg = max_deg;
+    g->rows = rows;
     g->loop_free = true;  // an undirected graph has no self-loop
     *out = g;
     return TC_OK;
@@ -782,7 +789,7 @@ int tc_graph_upload_i32(tc_ctx *ctx, const int32_t *row_ptr, const int32_t *col,
     if (st == TC_OK && nnz > 0 &&
         cudaMemcpyAsync(g->col, col, sizeof(int32_t) * (size_t)nnz, cudaMemcpyHostToDevice, s) != cudaSuccess)
         st = set_error(TC_E_CUDA, "col upload failed");
-    if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->max_deg);
+    if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->rows);
     if (st != TC_OK) {
         tc_graph_destroy(g);
         return st;
@@ -824,7 +831,7 @@ int tc_graph_upload_u64(tc_ctx *ctx, const uint64_t *row_ptr, const uint64_t *co
                         cudaStreamSynchronize(s) != cudaSuccess))
         st = set_error(TC_E_CUDA, "u64 narrowing failed");
     if (st == TC_OK && h_ovf) st = set_error(TC_E_RANGE, "u64 CSR value does not fit int32");
-    if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->max_deg);
+    if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->rows);
     if (st != TC_OK) {
         tc_graph_destroy(g);
         return st;
@@ -1245,7 +1252,7 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
                             cudaStreamSynchronize(Vs) != cudaSuccess))
             st = set_error(TC_E_CUDA, "validation failed to run");
         for (int p = 0; p < n_parts && st == TC_OK; ++p) {
-            st = validate_verdict(hv[(size_t)p], n_rows[p], nnz[p], &gs[(size_t)p]->max_deg);
+            st = validate_verdict(hv[(size_t)p], n_rows[p], nnz[p], &gs[(size_t)p]->rows);
             if (st != TC_OK) set_error(st, "part %d: %s", p, std::string(tc_last_error()).c_str());
             else if (cudaStreamWaitEvent(S, copied[(size_t)p], 0) != cudaSuccess)
                 st = set_error(TC_E_CUDA, "event wait failed");
@@ -1259,7 +1266,7 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
         if (st == TC_OK && (cudaMemcpyAsync(&h, d_err.p, sizeof h, cudaMemcpyDeviceToHost, Vs) != cudaSuccess ||
                             cudaStreamSynchronize(Vs) != cudaSuccess))
             st = set_error(TC_E_CUDA, "part %d: validation failed to run", p);
-        if (st == TC_OK) st = validate_verdict(h, n_rows[p], nnz[p], &g->max_deg);
+        if (st == TC_OK) st = validate_verdict(h, n_rows[p], nnz[p], &g->rows);
         if (st != TC_OK) {
             set_error(st, "part %d: %s", p, std::string(tc_last_error()).c_str());
             break;

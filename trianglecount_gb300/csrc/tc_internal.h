@@ -226,6 +226,39 @@ int radix_sort_u64(uint64_t **keys, uint64_t **tmp, int64_t n, int bits, cudaStr
 
 int device_sm_count(int device);
 
+// ---- row lengths (tc_api.cu) --------------------------------------------------------
+// What the choice of a graph's count asks of its rows' lengths.
+constexpr int64_t kSkew = 5;
+struct RowStats {
+    int32_t longest = -1;  // the longest row; -1: not known
+    uint32_t skewed = 0;   // entries in rows longer than kSkew x the mean (skew_bound)
+};
+inline int32_t skew_bound(int64_t n_rows, int64_t nnz) {
+    const int64_t b = n_rows > 0 ? kSkew * nnz / n_rows : 0;
+    return b < INT32_MAX ? (int32_t)b : INT32_MAX;
+}
+#ifdef __CUDACC__
+// One thread's rows, then a warp's added to the launch's (all lanes call add).
+struct RowTally {
+    int longest = 0;
+    unsigned skewed = 0;
+    __device__ __forceinline__ void row(int d, int skew) {
+        longest = max(longest, d);
+        if (d > skew) skewed += (unsigned)d;
+    }
+    __device__ __forceinline__ void add(RowStats *out) {
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        skewed = __reduce_add_sync(0xffffffffu, skewed);
+        if ((threadIdx.x & 31) == 0 && longest) {
+            atomicMax(&out->longest, longest);
+            if (skewed) atomicAdd(&out->skewed, skewed);
+        }
+    }
+};
+#endif
+// The row statistics of a device CSR into *d_out.
+int row_stats(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int64_t nnz, RowStats *d_out);
+
 // Counts n graphs (same device) with one batched launch on ctx's stream and
 // waits up to timeout_ms for the results (TC_E_TIMEOUT after that; the
 // launch is then still in flight).  Scratch comes from the stream-ordered pool.
@@ -268,7 +301,7 @@ struct tc_graph {
     int32_t *rp = nullptr;
     int32_t *col = nullptr;
     int64_t n_rows = 0, nnz = 0, n_roots = 0;
-    int32_t max_deg = -1;  // longest row, when known (uploads and device-built graphs)
+    tc::RowStats rows;     // known for uploads and device-built graphs
     bool owns = true;
     bool loop_free = false;  // no row holds its own id (device-built graphs)
     // per-graph count scratch, sized on first use

@@ -26,10 +26,8 @@
 namespace tc {
 
 int validate_csr(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_t n_rows, int64_t nnz);
-// Longest row (the out-degree bound that selects the flat count) into *d_out.
-int longest_row(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int32_t *d_out);
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       int32_t max_deg, tc_graph **out);
+                       const RowStats &rows, tc_graph **out);
 
 namespace {
 
@@ -576,13 +574,13 @@ __global__ void peel_round_kernel(int32_t *front_a, int32_t *front_b, int32_t *f
 }
 
 // Local ids (part vertices, then the halo that is left, each ascending) from the
-// scan of both (scan_halo_ids), -1 for the others; row lengths by local id; the
-// longest row.
+// scan of both (scan_halo_ids), -1 for the others; row lengths by local id and
+// their statistics (skew: the whole graph's bound, whose rows a part's own are).
 __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__restrict__ removed,
                                 const int64_t *__restrict__ ids, const int32_t *__restrict__ cnt, int64_t V,
-                                int32_t *__restrict__ lid, int32_t *__restrict__ len, int32_t *longest) {
+                                int32_t *__restrict__ lid, int32_t *__restrict__ len, int skew, RowStats *rows) {
     const int t_ver = (int)(ids[V] & 0xffffffffll);
-    int most = 0;
+    RowTally t;
     GRID_STRIDE(v, V) {
         const int c = cd[v].x;
         int l = -1;
@@ -591,12 +589,17 @@ __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__re
         lid[v] = l;
         if (l >= 0) {
             len[l] = cnt[v];
-            most = max(most, cnt[v]);
+            t.row(cnt[v], skew);
         }
     }
-    most = __reduce_max_sync(kFull, most);
-    if ((threadIdx.x & 31) == 0 && most) atomicMax(longest, most);
+    t.add(rows);
 }
+
+// Device words of one part's extraction.
+struct HaloWords {
+    int32_t front[3];  // frontier sizes (peel_round_kernel)
+    RowStats rows;
+};
 
 // Pass 2 (strided): ranks each tile's P and H entries again from the stored
 // bits with warp ballots and writes every local edge at lrp[local row] + its
@@ -894,13 +897,13 @@ int tc_orient(tc_ctx *ctx, const tc_ugraph *ug, int tie, tc_graph **out) {
     } else {
         TC_CUDA(cudaMemsetAsync(orp.p, 0, sizeof(int32_t) * (size_t)(V + 1), s));
     }
-    DBuf<int32_t> d_longest;
-    int32_t longest = 0;
-    TC_TRY(d_longest.alloc(1, s));
-    TC_TRY(longest_row(ctx, orp.p, V, d_longest.p));
-    TC_TRY(d2h_scalar(&longest, d_longest.p, s));
+    DBuf<RowStats> d_rows;
+    RowStats rows;
+    TC_TRY(d_rows.alloc(1, s));
+    TC_TRY(row_stats(ctx, orp.p, V, m32, d_rows.p));
+    TC_TRY(d2h_scalar(&rows, d_rows.p, s));
     tc_graph *g = nullptr;
-    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, longest, &g));
+    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, rows, &g));
     orp.release();
     ocol.release();
     *out = g;
@@ -934,7 +937,8 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         if (part[v] < 0) return set_error(TC_E_RANGE, "part[%lld] = %d is negative", (long long)v, part[v]);
     const int64_t tiles = (nnz + kOTile - 1) / kOTile;
     const size_t nv = (size_t)std::max<int64_t>(V, 1);
-    DBuf<int32_t> dpart, lid, cnt, lrp, tile_cnt, tile_off, base_p, base_h, indeg, front, next, words;
+    DBuf<int32_t> dpart, lid, cnt, lrp, tile_cnt, tile_off, base_p, base_h, indeg, front, next;
+    DBuf<HaloWords> words;
     DBuf<int64_t> ids;
     DBuf<int2> cd;
     DBuf<uint32_t> bits, mask;
@@ -953,7 +957,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
     TC_TRY(removed.alloc(nv, s));
     TC_TRY(front.alloc(nv, s));
     TC_TRY(next.alloc(nv, s));
-    TC_TRY(words.alloc(4, s));  // three frontier sizes, the longest row
+    TC_TRY(words.alloc(1, s));
     TC_TRY(row_rank.alloc((size_t)V + 1, s));
     TC_TRY(bits.alloc((size_t)std::max<int64_t>(tiles, 1) * kOT, s));
     TC_TRY(tile_cnt.alloc((size_t)std::max<int64_t>(3 * tiles, 1), s));
@@ -973,7 +977,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         TC_TRY(inH.alloc(nv, s));
     }
     struct Back {  // what the host reads per part
-        int32_t words[4];
+        HaloWords words;
         int64_t ids;
         int32_t nnz;
     } *back = (Back *)ctx->h_pinned;
@@ -990,7 +994,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             if (V) flag_class_kernel<<<gV, 256, 0, s>>>(inP.p, inH.p, ug->deg, V, cd.p);
         }
         TC_CUDA(cudaGetLastError());
-        TC_CUDA(cudaMemsetAsync(words.p, 0, 4 * sizeof(int32_t), s));
+        TC_CUDA(cudaMemsetAsync(words.p, 0, sizeof(HaloWords), s));
         if (tiles) {
             halo_tile_count_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, cd.p, nnz, V, tiles, tie, bits.p,
                                                                     tile_cnt.p, row_rank.p);
@@ -998,7 +1002,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             TC_TRY(scan_exclusive_i32(tile_cnt.p, tile_off.p, 3 * tiles, s));
             if (V)
                 halo_rows_kernel<<<gV, 256, 0, s>>>(ug->rp, cd.p, row_rank.p, tile_off.p, V, tiles, cnt.p, base_p.p,
-                                                    base_h.p, indeg.p, removed.p, front.p, words.p);
+                                                    base_h.p, indeg.p, removed.p, front.p, words.p->front);
             TC_CUDA(cudaGetLastError());
         } else {
             TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * nv, s));
@@ -1011,7 +1015,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         int round = 0;
         auto peel = [&](int n) {
             for (; n > 0 && tiles && !in_only; --n, ++round)
-                peel_round_kernel<<<ctx->sm_count * 8, 256, 0, s>>>(front.p, next.p, words.p, round, ug->rp, ug->col,
+                peel_round_kernel<<<ctx->sm_count * 8, 256, 0, s>>>(front.p, next.p, words.p->front, round, ug->rp, ug->col,
                                                                     cd.p, tie, indeg.p, removed.p);
         };
         peel(8);
@@ -1019,18 +1023,20 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         for (;; peel(4)) {
             TC_TRY(scan_halo_ids(cd.p, removed.p, ids.p, V, s));
             TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
-            TC_CUDA(cudaMemsetAsync(words.p + 3, 0, sizeof(int32_t), s));
-            if (V) halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, words.p + 3);
+            TC_CUDA(cudaMemsetAsync(&words.p->rows, 0, sizeof(RowStats), s));
+            if (V)
+                halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, skew_bound(V, nnz / 2),
+                                                   &words.p->rows);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
-            TC_CUDA(cudaMemcpyAsync(back->words, words.p, sizeof(back->words), cudaMemcpyDeviceToHost, s));
+            TC_CUDA(cudaMemcpyAsync(&back->words, words.p, sizeof(HaloWords), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaMemcpyAsync(&back->ids, ids.p + V, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaMemcpyAsync(&back->nnz, lrp.p + V, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaStreamSynchronize(s));
-            if (in_only || back->words[round % 3] == 0) break;
+            if (in_only || back->words.front[round % 3] == 0) break;
         }
         const int32_t t_ver = (int32_t)(back->ids & 0xffffffffll), n_halo = (int32_t)(back->ids >> 32);
-        const int32_t longest = back->words[3];
+        const RowStats rows = back->words.rows;
         const int64_t n_local = (int64_t)t_ver + n_halo, lnnz = back->nnz;
         DBuf<int32_t> rp, lcol;
         TC_TRY(rp.alloc((size_t)n_local + 1, s));
@@ -1040,7 +1046,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             halo_tile_write_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, lid.p, bits.p, nnz, tiles,
                                                                     tile_off.p, lrp.p, base_p.p, base_h.p, lcol.p);
         TC_CUDA(cudaGetLastError());
-        const int ast = graph_adopt_device(ctx, rp.p, lcol.p, n_local, lnnz, t_ver, longest, &parts_out[p]);
+        const int ast = graph_adopt_device(ctx, rp.p, lcol.p, n_local, lnnz, t_ver, rows, &parts_out[p]);
         if (ast == TC_OK) {
             rp.release();
             lcol.release();
