@@ -83,3 +83,31 @@ def test_skewed_graphs_count_packed(ctx, maker):
     parts = ctx.halo_extract(ug, gen.parts_random(ug.info()[0], 3), 3, mode="count")
     assert [ctx.count(p, stats=True)[1]["launches"] for p in parts] == [PACKED] * 3
     assert sum(ctx.count(p) for p in parts) == oracle.count(rp, col)
+
+
+@pytest.mark.parametrize("maker", ["chung_lu", "rmat18"])
+@pytest.mark.parametrize("order", ["ids", "descending"])
+def test_edges_that_do_not_go_by_degree_count_on_plain_ids(ctx, maker, order):
+    """Rows of thousands of unpopular ids; alone, and in a launch with as many other edges."""
+    n, (src, dst) = (100_000, gen.chung_lu(100_000, 16.0, seed=2)) if maker == "chung_lu" else (1 << 18, gen.rmat(18))
+    if order == "ids":
+        rank = np.random.default_rng(1).permutation(n)
+    else:
+        rank = -(np.bincount(np.concatenate((src, dst)), minlength=n).astype(np.int64) * n + np.arange(n))
+    rp, col = by_rank(n, src, dst, rank)
+    assert launches_of(ctx, rp, col) > PACKED
+    ordered = by_degree(n, src, dst)
+    assert launches_of(ctx, *ordered) == PACKED
+    b = ctx.batch([ctx.upload(rp, col), ctx.upload(*ordered), ctx.upload(*ordered)])
+    assert list(b.run()) == [oracle.count(rp, col)] + [oracle.count(*ordered)] * 2
+    assert b.stats()["launches"] > PACKED
+
+
+def test_a_small_share_of_such_a_graph_leaves_a_launch_packed(ctx):
+    n = 70_000
+    far = by_rank(n, *gen.chung_lu(n, 4.0, seed=2), np.random.default_rng(1).permutation(n))
+    rp, col = oracle.pipeline(*gen.rmat(18))[:2]
+    assert 16 * len(far[1]) < len(col)
+    b = ctx.batch([ctx.upload(*far), ctx.upload(rp, col)])
+    assert list(b.run()) == [oracle.count(*far), oracle.count(rp, col)]
+    assert b.stats()["launches"] == PACKED

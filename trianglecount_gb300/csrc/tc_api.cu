@@ -27,9 +27,9 @@ struct ValidateErr {
     int first;      // smallest offending row / entry index
     RowStats rows;  // of valid rows
 };
-constexpr ValidateErr kNoErr{0, 0x7fffffff, {0, 0}};
+constexpr ValidateErr kNoErr{0, 0x7fffffff, {0, 0, 0}};
 
-__global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz, int skew, uint8_t *start,
+__global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz, RowBounds bounds, uint8_t *start,
                                  ValidateErr *err) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     RowTally t;
@@ -41,17 +41,17 @@ __global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz,
             atomicMin(&err->first, (int)u);
         } else if (a < b) {
             start[a] = 1;
-            t.row((int)(b - a), skew);
+            t.row((int)(b - a), bounds);
         }
     }
     t.add(&err->rows);
 }
 
-__global__ void row_stats_kernel(const int32_t *rp, int64_t n_rows, int skew, RowStats *out) {
+__global__ void row_stats_kernel(const int32_t *rp, int64_t n_rows, RowBounds bounds, RowStats *out) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     RowTally t;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n_rows; u += stride)
-        t.row(rp[u + 1] - rp[u], skew);
+        t.row(rp[u + 1] - rp[u], bounds);
     t.add(out);
 }
 
@@ -112,7 +112,7 @@ int validate_csr_impl(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_
     const ValidateErr init = kNoErr;
     TC_CUDA(cudaMemcpyAsync(err.p, &init, sizeof(init), cudaMemcpyHostToDevice, s));
     if (n_rows > 0) {
-        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, skew_bound(n_rows, nnz), start.p,
+        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, row_bounds(n_rows, nnz), start.p,
                                                                          err.p);
         TC_CUDA(cudaGetLastError());
     }
@@ -143,7 +143,7 @@ int validate_csr_enqueue(tc_ctx *ctx, cudaStream_t s, const int32_t *rp, const i
     set_validate_err_kernel<<<1, 1, 0, s>>>(d_err, kNoErr);
     TC_CUDA(cudaGetLastError());
     if (n_rows > 0) {
-        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, skew_bound(n_rows, nnz), start,
+        mark_rows_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, s>>>(rp, n_rows, nnz, row_bounds(n_rows, nnz), start,
                                                                          d_err);
         TC_CUDA(cudaGetLastError());
     }
@@ -260,18 +260,26 @@ bool flat_count(const tc_graph *g) {
 // R-MAT graphs have 0.36 to 0.58 of their entries in such rows, Chung-Lu graphs
 // 0.08 to 0.26; an Erdos-Renyi graph of 8 M edges with a tenth of its edges in
 // cliques of 60 has 0.06 (0.67 ms plain, 0.76 packed).  One long row says nothing.
-constexpr int64_t kSkewShare = 16, kPackRows = 61440;
+//   A graph whose edges do not go by degree (an uploaded CSR may go by ids) has
+// rows of thousands, and the high blocks of a row are looked up a tile at a time,
+// all its lists streamed once per tile: Chung-Lu n = 1 M of mean degree 16 in random order
+// 1.3 ms plain, 7.7 packed (0.90 and 0.62 by degree), R-MAT 20 7.6 and 20.5.  So
+// graphs with 1 / kFarShare of their entries in such rows count on plain ids, and
+// so does a launch with as many of its entries in such graphs.
+constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440;
 bool skewed(const tc_graph *g) { return g->rows.longest < 0 || kSkewShare * g->rows.skewed >= g->nnz; }
+bool far_rows(const tc_graph *g) { return g->rows.far > 0 && kFarShare * g->rows.far >= g->nnz; }
 bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     if (!packed_count(tn)) return false;
-    int64_t V = 0, E = 0, gain = 0;
+    int64_t V = 0, E = 0, gain = 0, far = 0;
     for (int i = 0; i < n; ++i) {
         const tc_graph *g = gs[i];
-        if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
+        if (g->n_rows > kPackRows && far_rows(g)) far += g->nnz;
+        else if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
         V += g->n_rows + 1;
         E += g->nnz;
     }
-    return 2 * gain >= E && pack_fits(V, E);
+    return 2 * gain >= E && kFarShare * far <= E && pack_fits(V, E);
 }
 bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
 
@@ -601,7 +609,7 @@ int device_sm_count(int device) {
 int row_stats(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int64_t nnz, RowStats *d_out) {
     TC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(RowStats), ctx->stream));
     if (n_rows > 0)
-        row_stats_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, skew_bound(n_rows, nnz),
+        row_stats_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, row_bounds(n_rows, nnz),
                                                                                    d_out);
     TC_CUDA(cudaGetLastError());
     return TC_OK;

@@ -231,27 +231,38 @@ int device_sm_count(int device);
 constexpr int64_t kSkew = 5;
 struct RowStats {
     int32_t longest = -1;  // the longest row; -1: not known
-    uint32_t skewed = 0;   // entries in rows longer than kSkew x the mean (skew_bound)
+    uint32_t skewed = 0;   // entries in rows longer than kSkew x the mean
+    uint32_t far = 0;      // entries in rows that no degree orientation has (RowBounds)
 };
-inline int32_t skew_bound(int64_t n_rows, int64_t nnz) {
+// An orientation by degree has rows of at most sqrt(2 nnz) members, and in R-MAT
+// and Chung-Lu graphs of at most a tenth of that.
+struct RowBounds {
+    int32_t skew, far;
+};
+inline RowBounds row_bounds(int64_t n_rows, int64_t nnz) {
     const int64_t b = n_rows > 0 ? kSkew * nnz / n_rows : 0;
-    return b < INT32_MAX ? (int32_t)b : INT32_MAX;
+    int64_t f = 512;
+    while (16 * f * f < nnz) f += f / 8;  // about sqrt(nnz) / 4
+    return {b < INT32_MAX ? (int32_t)b : INT32_MAX, (int32_t)f};
 }
 #ifdef __CUDACC__
 // One thread's rows, then a warp's added to the launch's (all lanes call add).
 struct RowTally {
     int longest = 0;
-    unsigned skewed = 0;
-    __device__ __forceinline__ void row(int d, int skew) {
+    unsigned skewed = 0, far = 0;
+    __device__ __forceinline__ void row(int d, RowBounds b) {
         longest = max(longest, d);
-        if (d > skew) skewed += (unsigned)d;
+        if (d > b.skew) skewed += (unsigned)d;
+        if (d > b.far) far += (unsigned)d;
     }
     __device__ __forceinline__ void add(RowStats *out) {
         longest = __reduce_max_sync(0xffffffffu, longest);
         skewed = __reduce_add_sync(0xffffffffu, skewed);
+        far = __reduce_add_sync(0xffffffffu, far);
         if ((threadIdx.x & 31) == 0 && longest) {
             atomicMax(&out->longest, longest);
             if (skewed) atomicAdd(&out->skewed, skewed);
+            if (far) atomicAdd(&out->far, far);
         }
     }
 };

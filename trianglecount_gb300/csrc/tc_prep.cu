@@ -575,10 +575,10 @@ __global__ void peel_round_kernel(int32_t *front_a, int32_t *front_b, int32_t *f
 
 // Local ids (part vertices, then the halo that is left, each ascending) from the
 // scan of both (scan_halo_ids), -1 for the others; row lengths by local id and
-// their statistics (skew: the whole graph's bound, whose rows a part's own are).
+// their statistics (by the whole graph's bounds: a part's own rows are its rows).
 __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__restrict__ removed,
                                 const int64_t *__restrict__ ids, const int32_t *__restrict__ cnt, int64_t V,
-                                int32_t *__restrict__ lid, int32_t *__restrict__ len, int skew, RowStats *rows) {
+                                int32_t *__restrict__ lid, int32_t *__restrict__ len, RowBounds bounds, RowStats *rows) {
     const int t_ver = (int)(ids[V] & 0xffffffffll);
     RowTally t;
     GRID_STRIDE(v, V) {
@@ -589,7 +589,7 @@ __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__re
         lid[v] = l;
         if (l >= 0) {
             len[l] = cnt[v];
-            t.row(cnt[v], skew);
+            t.row(cnt[v], bounds);
         }
     }
     t.add(rows);
@@ -1025,7 +1025,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
             TC_CUDA(cudaMemsetAsync(&words.p->rows, 0, sizeof(RowStats), s));
             if (V)
-                halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, skew_bound(V, nnz / 2),
+                halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, row_bounds(V, nnz / 2),
                                                    &words.p->rows);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
