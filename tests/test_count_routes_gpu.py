@@ -111,3 +111,34 @@ def test_a_small_share_of_such_a_graph_leaves_a_launch_packed(ctx):
     b = ctx.batch([ctx.upload(*far), ctx.upload(rp, col)])
     assert list(b.run()) == [oracle.count(*far), oracle.count(rp, col)]
     assert b.stats()["launches"] == PACKED
+
+
+@pytest.mark.parametrize("maker", ["rmat20", "chung_lu"])
+def test_a_few_roots_of_a_large_graph_count_on_plain_ids(ctx, maker):
+    """The packed count packs every row, whether a root holds it or not."""
+    src, dst = gen.rmat(20) if maker == "rmat20" else gen.chung_lu(1_000_000, 16.0, seed=1)
+    rp, col, _ = oracle.pipeline(src, dst)
+    assert launches_of(ctx, rp, col, 300_000) == PACKED
+    for n_roots in (1, 2000):
+        assert launches_of(ctx, rp, col, n_roots) > PACKED
+    g = ctx.upload(rp.astype(np.uint64), col.astype(np.uint64), n_roots=2000)
+    assert ctx.count(g, stats=True)[1]["launches"] > PACKED
+    ug = ctx.ugraph_from_edges(src, dst)  # a small part and its halo
+    part = np.ones(ug.info()[0], np.int32)
+    part[::400] = 0
+    small, large = ctx.halo_extract(ug, part, 2)
+    whole = oracle.count(rp, col)
+    (a, sa), (b, sb) = ctx.count(small, stats=True), ctx.count(large, stats=True)
+    assert a + b == whole and sb["launches"] == PACKED
+    of_roots = int(small.download()[0][small.n_roots])
+    assert (sa["launches"] > PACKED) == (of_roots + (1 << 18) < small.nnz // 16 + (small.n_rows + 1) // 4)
+
+
+def test_few_edges_among_many_rows_count_on_plain_ids(ctx):
+    rp, col, _ = oracle.pipeline(*gen.rmat(16))
+
+    def among(n_rows):
+        return np.concatenate((rp, np.full(n_rows + 1 - len(rp), rp[-1], np.int32)))
+
+    assert launches_of(ctx, among(2_000_000), col) == PACKED
+    assert launches_of(ctx, among(8_000_000), col) > PACKED

@@ -266,20 +266,29 @@ bool flat_count(const tc_graph *g) {
 // 1.3 ms plain, 7.7 packed (0.90 and 0.62 by degree), R-MAT 20 7.6 and 20.5.  So
 // graphs with 1 / kFarShare of their entries in such rows count on plain ids, and
 // so does a launch with as many of its entries in such graphs.
-constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440;
+//   Every row is packed, also the rows that no root holds, and every row, empty or
+// not, is looked at by four passes: a few roots of a large graph, or few edges
+// among many rows, do not pay for that.  R-MAT 20 (16 M edges) counts 0.12 / 0.48 /
+// 1.2 M root edges in 0.35 / 0.31 / 0.36 ms packed, 0.25 / 0.35 / 0.51 plain;
+// Chung-Lu n = 1 M (8 M edges) 0.39 / 0.79 M in 0.25 / 0.26 and 0.22 / 0.27;
+// R-MAT 16 (0.9 M edges) in 4 / 8 M rows 0.28 / 0.48 and 0.33 / 0.39, R-MAT 19
+// (7.7 M) in 16 / 32 M rows 1.24 / 2.07 and 1.68 / 1.98.  Graphs of any of these
+// shapes with fewer than 2^18 edges and rows gain from the fewer launches.
+constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440, kPackFree = 1 << 18;
 bool skewed(const tc_graph *g) { return g->rows.longest < 0 || kSkewShare * g->rows.skewed >= g->nnz; }
 bool far_rows(const tc_graph *g) { return g->rows.far > 0 && kFarShare * g->rows.far >= g->nnz; }
 bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     if (!packed_count(tn)) return false;
-    int64_t V = 0, E = 0, gain = 0, far = 0;
+    int64_t V = 0, E = 0, gain = 0, far = 0, of_roots = kPackFree;
     for (int i = 0; i < n; ++i) {
         const tc_graph *g = gs[i];
         if (g->n_rows > kPackRows && far_rows(g)) far += g->nnz;
         else if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
+        of_roots += g->root_nnz >= 0 ? g->root_nnz : g->nnz;
         V += g->n_rows + 1;
         E += g->nnz;
     }
-    return 2 * gain >= E && kFarShare * far <= E && pack_fits(V, E);
+    return 2 * gain >= E && kFarShare * far <= E && of_roots >= E / 16 + V / 4 && pack_fits(V, E);
 }
 bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
 
@@ -616,13 +625,14 @@ int row_stats(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int64_t nnz, RowSt
 }
 
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       const RowStats &rows, tc_graph **out) {
+                       int64_t root_nnz, const RowStats &rows, tc_graph **out) {
     tc_graph *g = nullptr;
     TC_TRY(new_graph(ctx, n_rows, nnz, n_roots, &g));
     g->rp = rp;
     g->col = col;
     g->owns = true;
     g->rows = rows;
+    g->root_nnz = root_nnz;
     g->loop_free = true;  // an undirected graph has no self-loop
     *out = g;
     return TC_OK;
@@ -798,6 +808,7 @@ int tc_graph_upload_i32(tc_ctx *ctx, const int32_t *row_ptr, const int32_t *col,
         cudaMemcpyAsync(g->col, col, sizeof(int32_t) * (size_t)nnz, cudaMemcpyHostToDevice, s) != cudaSuccess)
         st = set_error(TC_E_CUDA, "col upload failed");
     if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->rows);
+    g->root_nnz = st == TC_OK ? (int64_t)row_ptr[n_roots] : -1;
     if (st != TC_OK) {
         tc_graph_destroy(g);
         return st;
@@ -840,6 +851,7 @@ int tc_graph_upload_u64(tc_ctx *ctx, const uint64_t *row_ptr, const uint64_t *co
         st = set_error(TC_E_CUDA, "u64 narrowing failed");
     if (st == TC_OK && h_ovf) st = set_error(TC_E_RANGE, "u64 CSR value does not fit int32");
     if (st == TC_OK) st = validate_csr_impl(ctx, g->rp, g->col, n_rows, nnz, &g->rows);
+    g->root_nnz = st == TC_OK ? (int64_t)row_ptr[n_roots] : -1;
     if (st != TC_OK) {
         tc_graph_destroy(g);
         return st;
@@ -1261,6 +1273,7 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
             st = set_error(TC_E_CUDA, "validation failed to run");
         for (int p = 0; p < n_parts && st == TC_OK; ++p) {
             st = validate_verdict(hv[(size_t)p], n_rows[p], nnz[p], &gs[(size_t)p]->rows);
+            gs[(size_t)p]->root_nnz = row_ptrs[p][n_roots[p]];
             if (st != TC_OK) set_error(st, "part %d: %s", p, std::string(tc_last_error()).c_str());
             else if (cudaStreamWaitEvent(S, copied[(size_t)p], 0) != cudaSuccess)
                 st = set_error(TC_E_CUDA, "event wait failed");
@@ -1275,6 +1288,7 @@ int tc_count_parts_csr_i32(tc_ctx *ctx, int n_parts, const int32_t *const *row_p
                             cudaStreamSynchronize(Vs) != cudaSuccess))
             st = set_error(TC_E_CUDA, "part %d: validation failed to run", p);
         if (st == TC_OK) st = validate_verdict(h, n_rows[p], nnz[p], &g->rows);
+        g->root_nnz = row_ptrs[p][n_roots[p]];
         if (st != TC_OK) {
             set_error(st, "part %d: %s", p, std::string(tc_last_error()).c_str());
             break;

@@ -313,6 +313,7 @@ struct tc_graph {
     int32_t *col = nullptr;
     int64_t n_rows = 0, nnz = 0, n_roots = 0;
     tc::RowStats rows;     // known for uploads and device-built graphs
+    int64_t root_nnz = -1; // entries in the roots' rows; -1: not known
     bool owns = true;
     bool loop_free = false;  // no row holds its own id (device-built graphs)
     // per-graph count scratch, sized on first use

@@ -19,6 +19,7 @@
 // each ascending) -> scan of the row lengths -> ordered write of every local
 // edge, once.
 #include <algorithm>
+#include <cstddef>
 #include <vector>
 
 #include "tc_internal.h"
@@ -27,7 +28,7 @@ namespace tc {
 
 int validate_csr(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_t n_rows, int64_t nnz);
 int graph_adopt_device(tc_ctx *ctx, int32_t *rp, int32_t *col, int64_t n_rows, int64_t nnz, int64_t n_roots,
-                       const RowStats &rows, tc_graph **out);
+                       int64_t root_nnz, const RowStats &rows, tc_graph **out);
 
 namespace {
 
@@ -573,14 +574,22 @@ __global__ void peel_round_kernel(int32_t *front_a, int32_t *front_b, int32_t *f
     }
 }
 
+// Device words of one part's extraction.
+struct HaloWords {
+    int32_t front[3];  // frontier sizes (peel_round_kernel)
+    int32_t root_nnz;  // entries in the rows of the part's vertices
+    RowStats rows;
+};
+
 // Local ids (part vertices, then the halo that is left, each ascending) from the
 // scan of both (scan_halo_ids), -1 for the others; row lengths by local id and
 // their statistics (by the whole graph's bounds: a part's own rows are its rows).
 __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__restrict__ removed,
                                 const int64_t *__restrict__ ids, const int32_t *__restrict__ cnt, int64_t V,
-                                int32_t *__restrict__ lid, int32_t *__restrict__ len, RowBounds bounds, RowStats *rows) {
+                                int32_t *__restrict__ lid, int32_t *__restrict__ len, RowBounds bounds, HaloWords *words) {
     const int t_ver = (int)(ids[V] & 0xffffffffll);
     RowTally t;
+    int of_roots = 0;
     GRID_STRIDE(v, V) {
         const int c = cd[v].x;
         int l = -1;
@@ -590,16 +599,13 @@ __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__re
         if (l >= 0) {
             len[l] = cnt[v];
             t.row(cnt[v], bounds);
+            if (c == 0) of_roots += cnt[v];
         }
     }
-    t.add(rows);
+    t.add(&words->rows);
+    of_roots = __reduce_add_sync(kFull, of_roots);
+    if ((threadIdx.x & 31) == 0 && of_roots) atomicAdd(&words->root_nnz, of_roots);
 }
-
-// Device words of one part's extraction.
-struct HaloWords {
-    int32_t front[3];  // frontier sizes (peel_round_kernel)
-    RowStats rows;
-};
 
 // Pass 2 (strided): ranks each tile's P and H entries again from the stored
 // bits with warp ballots and writes every local edge at lrp[local row] + its
@@ -903,7 +909,7 @@ int tc_orient(tc_ctx *ctx, const tc_ugraph *ug, int tie, tc_graph **out) {
     TC_TRY(row_stats(ctx, orp.p, V, m32, d_rows.p));
     TC_TRY(d2h_scalar(&rows, d_rows.p, s));
     tc_graph *g = nullptr;
-    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, rows, &g));
+    TC_TRY(graph_adopt_device(ctx, orp.p, ocol.p, V, m32, V, m32, rows, &g));
     orp.release();
     ocol.release();
     *out = g;
@@ -1023,10 +1029,10 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         for (;; peel(4)) {
             TC_TRY(scan_halo_ids(cd.p, removed.p, ids.p, V, s));
             TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
-            TC_CUDA(cudaMemsetAsync(&words.p->rows, 0, sizeof(RowStats), s));
+            TC_CUDA(cudaMemsetAsync(&words.p->root_nnz, 0, sizeof(HaloWords) - offsetof(HaloWords, root_nnz), s));
             if (V)
                 halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, row_bounds(V, nnz / 2),
-                                                   &words.p->rows);
+                                                   words.p);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
             TC_CUDA(cudaMemcpyAsync(&back->words, words.p, sizeof(HaloWords), cudaMemcpyDeviceToHost, s));
@@ -1046,7 +1052,8 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             halo_tile_write_kernel<<<(unsigned)tiles, kOT, 0, s>>>(ug->rowid, ug->col, lid.p, bits.p, nnz, tiles,
                                                                     tile_off.p, lrp.p, base_p.p, base_h.p, lcol.p);
         TC_CUDA(cudaGetLastError());
-        const int ast = graph_adopt_device(ctx, rp.p, lcol.p, n_local, lnnz, t_ver, rows, &parts_out[p]);
+        const int ast = graph_adopt_device(ctx, rp.p, lcol.p, n_local, lnnz, t_ver, back->words.root_nnz, rows,
+                                           &parts_out[p]);
         if (ast == TC_OK) {
             rp.release();
             lcol.release();
