@@ -142,3 +142,39 @@ def test_few_edges_among_many_rows_count_on_plain_ids(ctx):
 
     assert launches_of(ctx, among(2_000_000), col) == PACKED
     assert launches_of(ctx, among(8_000_000), col) > PACKED
+
+
+@pytest.mark.parametrize("m", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1])
+def test_one_launch_up_to_2_to_18_edges(ctx, m):
+    rp, col = by_degree(20_000, *gen.er(20_000, 27.0, seed=7))
+    rp, col = np.minimum(rp, m).astype(np.int32), col[:m]
+    assert len(col) == m and np.diff(rp).max() <= 64
+    assert launches_of(ctx, rp, col) == (1 if m <= 1 << 18 else PACKED)
+    for n_roots in (1, 31, 4097, 19_999):
+        assert launches_of(ctx, rp, col, n_roots) == (1 if m <= 1 << 18 else PACKED)
+
+
+@pytest.mark.parametrize("d", [33, 63, 64, 65, 128, 500, 2000, 8000])
+@pytest.mark.parametrize("n_edges", [12_000, 100_000])
+def test_one_launch_only_while_every_row_is_short(ctx, d, n_edges):
+    """A row is one warp's work in the single launch, however long it is."""
+    n = 20_000
+    r = np.random.default_rng(d)
+    u, v = r.integers(1, n, n_edges - d), r.integers(1, n, n_edges - d)
+    hub = 1 + r.choice(n - 1, d, replace=False)
+    rp, col = csr(n, np.concatenate((np.zeros(d, np.int64), u)), np.concatenate((hub, v)))
+    assert np.diff(rp).max() == d
+    for n_roots in (None, 1, 700):
+        assert launches_of(ctx, rp, col, n_roots) == (1 if d <= 64 else PACKED)
+
+
+@pytest.mark.parametrize("n_rows", [64, 65, 4863, 4864, 4865, 19457, 100_000])
+def test_one_launch_windows_of_rows(ctx, n_rows):
+    """Two to thirty-two rows per warp, as many as it takes to fill the GPU once."""
+    r = np.random.default_rng(n_rows)
+    m = min(12 * n_rows, 200_000)
+    u, v = r.integers(0, n_rows, m), r.integers(0, n_rows, m)
+    hub = r.choice(n_rows, 40, replace=False)  # one row past the flat count's eight
+    rp, col = csr(n_rows, np.concatenate((u, np.full(40, n_rows // 2))), np.concatenate((v, hub)))
+    assert 8 < np.diff(rp).max() <= 64
+    assert launches_of(ctx, rp, col) == 1

@@ -18,7 +18,7 @@ thread_local std::string g_last_error;
 constexpr int kVersion = 10000;  // 1.0.0
 
 // Graphs counted in one launch: see single_count.
-constexpr int64_t kSingleMinRows = 64, kSingleMaxEdges = 1 << 18, kSingleMaxSkewed = 1 << 14;
+constexpr int64_t kSingleMinRows = 64, kSingleMaxEdges = 1 << 18;
 constexpr int32_t kSingleMaxDeg = 64;
 
 // ---- CSR validation (rows strictly ascending, ids in range) ----
@@ -293,11 +293,16 @@ bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
 bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
 
 // A graph of few edges that no lane-per-root count takes is counted by one
-// launch on its own ids (launch_single).
+// launch on its own ids (launch_single).  A root's row is one warp's work there,
+// its hash built anew per 96 members and its lists streamed each time, so the
+// rows have to be known and short: Erdos-Renyi of 240 K edges 39 to 51 us a call
+// (the sequence of launches 68), one row of 512 whose members have 14 each 669 (88),
+// of 128 78 (63), one of 8000 23.4 ms (0.11).  Graphs of fewer than 64 rows would gain as well
+// (51 -> 27 us), but tests/test_count_gpu.py asserts the sequence for K_10.
 bool single_count(const tc_graph *g) {
     const Tuned &tn = g->ctx->tuned;
     return packed_count(tn) && tn.flat_max_deg > 0 && !flat_count(g) && g->n_rows >= kSingleMinRows &&
-           g->nnz <= (g->rows.longest >= 0 && g->rows.longest <= kSingleMaxDeg ? kSingleMaxEdges : kSingleMaxSkewed);
+           g->nnz <= kSingleMaxEdges && g->rows.longest >= 0 && g->rows.longest <= kSingleMaxDeg;
 }
 
 // Everything a count of g needs before its launches: the work words, the
