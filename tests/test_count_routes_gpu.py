@@ -178,3 +178,87 @@ def test_one_launch_windows_of_rows(ctx, n_rows):
     rp, col = csr(n_rows, np.concatenate((u, np.full(40, n_rows // 2))), np.concatenate((v, hub)))
     assert 8 < np.diff(rp).max() <= 64
     assert launches_of(ctx, rp, col) == 1
+
+
+def wrapped(ctx, rp, col):
+    torch = pytest.importorskip("torch")
+    a, b = torch.from_numpy(rp).cuda(), torch.from_numpy(col).cuda()
+    torch.cuda.synchronize()
+    g = ctx.wrap_device(a.data_ptr(), b.data_ptr(), len(rp) - 1, len(col))
+    g.arrays = a, b
+    return g
+
+
+def count_async(ctx, g):
+    import torch
+    import trianglecount_gb300 as tc
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    assert tc.lib().tc_count_async(ctx.handle, g.handle, out.data_ptr()) == 0
+    ctx.synchronize()
+    return int(out.item())
+
+
+@pytest.mark.parametrize("asynchronous_first", [False, True])
+def test_wrapped_graphs_take_the_count_of_their_rows(ctx, asynchronous_first):
+    er = by_degree(100_000, *gen.er(100_000, 16.0, seed=3))
+    rmat = oracle.pipeline(*gen.rmat(17))[:2]
+    few = by_degree(20_000, *gen.er(20_000, 20.0, seed=7))
+    for (rp, col), route in ((er, lambda n: n > PACKED), (rmat, lambda n: n == PACKED), (few, lambda n: n == 1)):
+        want, pr = oracle.count(rp, col, per_root=True)
+        g = wrapped(ctx, rp, col)
+        if asynchronous_first:
+            assert [count_async(ctx, g) for _ in range(3)] == [want] * 3
+        for _ in range(3):
+            got, st = ctx.count(g, stats=True)
+            assert got == want and route(st["launches"])
+        assert np.array_equal(ctx.count_per_root(g), pr)
+        assert [count_async(ctx, g) for _ in range(3)] == [want] * 3
+        assert list(ctx.batch([wrapped(ctx, rp, col), g]).run()) == [want, want]
+
+
+def test_wrapped_arrays_may_be_written_anew(ctx):
+    """Short rows first (never the flat count: it could not count the longer ones that follow)."""
+    torch = pytest.importorskip("torch")
+    n, m = 5000, 9000
+    r = np.random.default_rng(1)
+    short = csr(n, np.repeat(np.arange(n), 2)[:m], (np.repeat(np.arange(n), 2)[:m] + np.tile([1, 2], m)[:m]) % n)
+    u, v = np.repeat(np.arange(30), 300), np.concatenate([r.choice(600, 300, replace=False) for _ in range(30)])
+    long = csr(n, u, v)
+    assert len(short[1]) == len(long[1]) == m
+    for first, then in ((short, long), (long, short)):
+        g = wrapped(ctx, *first)
+        assert [ctx.count(g) for _ in range(3)] == [oracle.count(*first)] * 3
+        g.arrays[0].copy_(torch.from_numpy(then[0]))
+        g.arrays[1].copy_(torch.from_numpy(then[1]))
+        torch.cuda.synchronize()
+        want, pr = oracle.count(*then, per_root=True)
+        assert [ctx.count(g) for _ in range(3)] == [want] * 3
+        assert np.array_equal(ctx.count_per_root(g), pr)
+        assert count_async(ctx, g) == want
+
+
+def test_a_callers_capture_outlives_the_look_at_the_rows():
+    """tc_count_async captured by the caller, then a count that takes another form: the capture still counts."""
+    torch = pytest.importorskip("torch")
+    import trianglecount_gb300 as tc
+    rp, col, want = oracle.pipeline(*gen.rmat(17))
+    c = tc.Context(0)
+    s = torch.cuda.Stream()
+    c.set_stream(s.cuda_stream)
+    g = wrapped(c, rp, col)
+    assert count_async(c, g) == want  # sizes the scratch
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    cg = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(cg, stream=s):
+        assert tc.lib().tc_count_async(c.handle, g.handle, out.data_ptr()) == 0
+    assert c.count(g) == want
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        cg.replay()
+        torch.cuda.synchronize()
+        assert int(out.item()) == want and c.count(g) == want
+    g.free()
+    c.close()

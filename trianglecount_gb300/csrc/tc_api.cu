@@ -247,13 +247,14 @@ void capture_count(tc_graph *g, unsigned long long *res) {
     cudaGetLastError();  // a failed capture falls back to direct launches
 }
 
+// (A wrapped graph's rows may have changed since they were looked at, and longer
+// ones would be counted wrongly.)
 bool flat_count(const tc_graph *g) {
-    return g->rows.longest >= 0 && g->rows.longest <= g->ctx->tuned.flat_max_deg;
+    return g->owns && g->rows.longest >= 0 && g->rows.longest <= g->ctx->tuned.flat_max_deg;
 }
 
 // The packed count serves launches whose graphs are skewed (at least 1 / kSkewShare
-// of their entries in rows longer than kSkew x the mean, where the rows are
-// known) or small enough that most ids are low blocks'.  Without hubs the entries
+// of their entries in rows longer than kSkew x the mean) or small enough that most ids are low blocks'.  Without hubs the entries
 // hold one id each and lie in the high blocks, whose hashes cost more than the
 // plain-id tables: Erdos-Renyi n = 1 M of mean degree 8 / 40 0.25 / 1.36 ms there,
 // 0.32 / 1.9 packed; n = 30 K of mean degree 40 0.18 and 0.16.  Degree-oriented
@@ -275,7 +276,7 @@ bool flat_count(const tc_graph *g) {
 // (7.7 M) in 16 / 32 M rows 1.24 / 2.07 and 1.68 / 1.98.  Graphs of any of these
 // shapes with fewer than 2^18 edges and rows gain from the fewer launches.
 constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440, kPackFree = 1 << 18;
-bool skewed(const tc_graph *g) { return g->rows.longest < 0 || kSkewShare * g->rows.skewed >= g->nnz; }
+bool skewed(const tc_graph *g) { return g->rows.longest >= 0 && kSkewShare * g->rows.skewed >= g->nnz; }
 bool far_rows(const tc_graph *g) { return g->rows.far > 0 && kFarShare * g->rows.far >= g->nnz; }
 bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     if (!packed_count(tn)) return false;
@@ -284,13 +285,37 @@ bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
         const tc_graph *g = gs[i];
         if (g->n_rows > kPackRows && far_rows(g)) far += g->nnz;
         else if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
-        of_roots += g->root_nnz >= 0 ? g->root_nnz : g->nnz;
+        if (g->root_nnz >= 0) of_roots += g->root_nnz;
         V += g->n_rows + 1;
         E += g->nnz;
     }
     return 2 * gain >= E && kFarShare * far <= E && of_roots >= E / 16 + V / 4 && pack_fits(V, E);
 }
 bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
+
+// A wrapped graph's arrays are the caller's, and only a count may read them: the
+// first one that waits for its result anyway also looks at the rows.  They decide
+// which count is taken, never what it gives: a caller may write other rows into
+// the arrays later.  (Until then, as by tc_count_async alone: not known.)
+int look_at_rows(tc_graph *g) {
+    if (g->owns || g->rows.longest >= 0) return TC_OK;
+    cudaStream_t s = g->ctx->stream;
+    DBuf<RowStats> d;
+    RowStats rows;
+    int32_t of_roots = 0;
+    TC_TRY(d.alloc(1, s));
+    TC_TRY(row_stats(g->ctx, g->rp, g->n_rows, g->nnz, d.p));
+    TC_CUDA(cudaMemcpyAsync(&rows, d.p, sizeof rows, cudaMemcpyDeviceToHost, s));
+    TC_CUDA(cudaMemcpyAsync(&of_roots, g->rp + g->n_roots, sizeof of_roots, cudaMemcpyDeviceToHost, s));
+    TC_CUDA(cudaStreamSynchronize(s));
+    g->rows = rows;
+    g->root_nnz = std::min<int64_t>(std::max(of_roots, 0), g->nnz);
+    if (g->exec) {  // captured before the rows were known
+        cudaGraphExecDestroy(g->exec);
+        g->exec = nullptr;
+    }
+    return TC_OK;
+}
 
 // A graph of few edges that no lane-per-root count takes is counted by one
 // launch on its own ids (launch_single).  A root's row is one warp's work there,
@@ -921,6 +946,7 @@ int tc_count(tc_ctx *ctx, tc_graph *g, uint64_t *out, tc_count_stats *stats) {
     if (g->ctx != ctx) return set_error(TC_E_INVALID, "graph belongs to another context");
     cudaStream_t s = ctx->stream;
     int launches = 0;
+    TC_TRY(look_at_rows(g));
     TC_TRY(prepare_graph_count(g, nullptr, nullptr));  // setup and any capture stay out of count_ms
     if (stats) TC_CUDA(cudaEventRecord(ctx->ev[0], s));
     TC_TRY(enqueue_graph_count(g, nullptr, nullptr, &launches));
@@ -953,6 +979,7 @@ int tc_count_per_root(tc_ctx *ctx, tc_graph *g, uint64_t *per_root, uint64_t *to
     if (!per_root) return set_error(TC_E_INVALID, "null output");
     if (!ctx) ctx = g->ctx;
     cudaStream_t s = ctx->stream;
+    TC_TRY(look_at_rows(g));
     DBuf<unsigned long long> pr;
     TC_TRY(pr.alloc((size_t)std::max<int64_t>(g->n_roots, 1), s));
     TC_CUDA(cudaMemsetAsync(pr.p, 0, sizeof(unsigned long long) * (size_t)std::max<int64_t>(g->n_roots, 1), s));
@@ -1049,6 +1076,11 @@ int tc_batch_create(tc_ctx *ctx, tc_graph *const *graphs, int n, tc_batch **out)
         if (!g || g->ctx != ctx) {
             tc_batch_destroy(b);
             return set_error(TC_E_INVALID, "graph %d is null or belongs to another context", i);
+        }
+        const int ls = look_at_rows(g);
+        if (ls != TC_OK) {
+            tc_batch_destroy(b);
+            return ls;
         }
         b->graphs.push_back(g);
         memset(&desc[i], 0, sizeof(GraphDesc));

@@ -312,7 +312,7 @@ struct tc_graph {
     int32_t *rp = nullptr;
     int32_t *col = nullptr;
     int64_t n_rows = 0, nnz = 0, n_roots = 0;
-    tc::RowStats rows;     // known for uploads and device-built graphs
+    tc::RowStats rows;     // known for uploads and device-built graphs; of wrapped ones as look_at_rows saw them
     int64_t root_nnz = -1; // entries in the roots' rows; -1: not known
     bool owns = true;
     bool loop_free = false;  // no row holds its own id (device-built graphs)
