@@ -1015,8 +1015,10 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             TC_CUDA(cudaMemsetAsync(removed.p, 0, nv, s));
         }
         // Peel halo vertices of zero in-degree until none is left: eight rounds,
-        // then four more per look while there is a frontier (each round that has
-        // one removes a vertex).  A counting halo has none: each of its vertices
+        // then, while there is a frontier, more (each round that has one removes a
+        // vertex), twice as many per look up to 64.  Few halos need more than eight
+        // (the members are numbered without a look before), but a chain of n
+        // vertices needs n rounds.  A counting halo has none: each of its vertices
         // has an in-edge from the part.
         int round = 0;
         auto peel = [&](int n) {
@@ -1024,9 +1026,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
                 peel_round_kernel<<<ctx->sm_count * 8, 256, 0, s>>>(front.p, next.p, words.p->front, round, ug->rp, ug->col,
                                                                     cd.p, tie, indeg.p, removed.p);
         };
-        peel(8);
-        TC_CUDA(cudaGetLastError());
-        for (;; peel(4)) {
+        auto number = [&]() -> int {
             TC_TRY(scan_halo_ids(cd.p, removed.p, ids.p, V, s));
             TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
             TC_CUDA(cudaMemsetAsync(&words.p->root_nnz, 0, sizeof(HaloWords) - offsetof(HaloWords, root_nnz), s));
@@ -1035,11 +1035,27 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
                                                    words.p);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
-            TC_CUDA(cudaMemcpyAsync(&back->words, words.p, sizeof(HaloWords), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaMemcpyAsync(&back->ids, ids.p + V, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaMemcpyAsync(&back->nnz, lrp.p + V, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+            return TC_OK;
+        };
+        auto look = [&]() -> int {
+            TC_CUDA(cudaMemcpyAsync(&back->words, words.p, sizeof(HaloWords), cudaMemcpyDeviceToHost, s));
             TC_CUDA(cudaStreamSynchronize(s));
-            if (in_only || back->words.front[round % 3] == 0) break;
+            return TC_OK;
+        };
+        peel(8);
+        TC_CUDA(cudaGetLastError());
+        TC_TRY(number());
+        TC_TRY(look());
+        if (!in_only && back->words.front[round % 3] != 0) {
+            for (int more = 8; back->words.front[round % 3] != 0; more = std::min(64, 2 * more)) {
+                peel(more);
+                TC_CUDA(cudaGetLastError());
+                TC_TRY(look());
+            }
+            TC_TRY(number());
+            TC_TRY(look());
         }
         const int32_t t_ver = (int32_t)(back->ids & 0xffffffffll), n_halo = (int32_t)(back->ids >> 32);
         const RowStats rows = back->words.rows;
