@@ -103,8 +103,9 @@ __device__ __forceinline__ int lp_pick(const int32_t *h, int k, uint64_t seed, i
     return __shfl_sync(kFull, bl, __ffs(__ballot_sync(kFull, bl >= 0)) - 1);
 }
 
-// Per vertex, the label most common among its neighbours.  A block takes 256
-// consecutive vertices, a warp 32 of them.  With at most 16 parts, vertices of
+// Per vertex, the label most common among its neighbours.  A block takes eight
+// times per_warp consecutive vertices, a warp per_warp of them: 32, or fewer while
+// that many would leave SMs without a block (lp_per_warp).  With at most 16 parts, vertices of
 // degree <= 255 (kGroupDeg) are counted by eight lanes each, four at a time:
 // the counts are bytes packed in kWords 64-bit registers per lane and are
 // summed over the lanes with shuffles -- no histogram in memory, and the warp
@@ -118,8 +119,8 @@ constexpr int kGroupDeg = 255, kWarpDeg = 1024;
 template <int kWords>
 __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                         const uint8_t *__restrict__ label, int64_t n, int k,
-                                                        uint64_t seed, int it, int i_batch, LpIter *batch,
-                                                        int8_t *__restrict__ desired) {
+                                                        int per_warp, uint64_t seed, int it, int i_batch,
+                                                        LpIter *batch, int8_t *__restrict__ desired) {
     __shared__ int32_t hist[kPT / 32][kMaxParts];
     __shared__ int32_t s_flow[kMaxParts * kMaxParts];  // candidates from part a to part b at [a * k + b]
     __shared__ int s_big[kPT], s_nbig;
@@ -129,10 +130,12 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
     if (threadIdx.x == 0) s_nbig = 0;
     __syncthreads();
     int32_t *h = hist[warp];
-    for (int64_t v0 = (int64_t)blockIdx.x * kPT; v0 < n; v0 += (int64_t)gridDim.x * kPT) {
-        const int64_t mine = v0 + threadIdx.x;
+    const int per_block = per_warp * (kPT / 32), slot = warp * per_warp + lane;  // slot: a lane's vertex in its block
+    for (int64_t v0 = (int64_t)blockIdx.x * per_block; v0 < n; v0 += (int64_t)gridDim.x * per_block) {
+        const int64_t first = v0 + warp * per_warp, mine = first + lane;
+        const bool has = lane < per_warp && mine < n;
         int rs = 0, d = 0, cur = 0;
-        if (mine < n) {
+        if (has) {
             rs = rp[mine];
             d = rp[mine + 1] - rs;
             cur = label[mine];
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
         int choice = -1;  // of this lane's vertex
         if (kWords > 0) {
             const int g = lane >> 3, l8 = lane & 7;
-            for (int r = 0; r < 32; r += 4) {
+            for (int r = 0; r < per_warp; r += 4) {
                 const int src = r + g;  // the group's vertex: lane src's
                 const int a = __shfl_sync(kFull, rs, src);
                 const int dd = __shfl_sync(kFull, grouped ? d : 0, src), cl = __shfl_sync(kFull, cur, src);
@@ -183,7 +186,7 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
                             if (count[w] == best) {
                                 const int l = 8 * w + l8;
                                 const unsigned long long t =
-                                    ((unsigned long long)(hash_vl(seed, it, v0 + (threadIdx.x & ~31) + src, l) >> 1) << 8) |
+                                    ((unsigned long long)(hash_vl(seed, it, first + src, l) >> 1) << 8) |
                                     (unsigned long long)(255 - l);
                                 key = t > key ? t : key;
                             }
@@ -216,11 +219,11 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
                     if (q[i] >= 0) atomicAdd(&h[q[i]], 1);
             }
             __syncwarp();
-            const int pick = lp_pick(h, k, seed, it, v0 + (threadIdx.x & ~31) + src, cl, lane);
+            const int pick = lp_pick(h, k, seed, it, first + src, cl, lane);
             if (lane == src) choice = pick;
             __syncwarp();
         }
-        if (d > kWarpDeg && !grouped) s_big[atomicAdd(&s_nbig, 1)] = threadIdx.x;
+        if (d > kWarpDeg && !grouped) s_big[atomicAdd(&s_nbig, 1)] = slot;
         __syncthreads();
         const int nbig = s_nbig;
         for (int b = 0; b < nbig; ++b) {
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
             __syncthreads();
         }
         if (threadIdx.x == 0) s_nbig = 0;  // read by all before the last barrier above, or none was listed
-        if (mine < n && (grouped || d <= kWarpDeg)) {
+        if (has && (grouped || d <= kWarpDeg)) {
             desired[mine] = (int8_t)choice;
             if (choice >= 0) atomicAdd(&s_flow[cur * k + choice], 1);
         }
@@ -324,6 +327,14 @@ __global__ void lp_widen_kernel(const uint8_t *label, int64_t n, int32_t *out) {
         out[v] = label[v];
 }
 
+// Vertices per warp of the choose pass, at least four where a warp counts four at a
+// time.
+int lp_per_warp(int64_t n, int k, const tc_ctx *ctx) {
+    int w = 32;
+    while (w > (k <= 16 ? 4 : 1) && n / (w * (kPT / 32)) < (int64_t)ctx->sm_count * 4) w /= 2;
+    return w;
+}
+
 int pgrid(int64_t n, const tc_ctx *ctx) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kPT - 1) / kPT, (int64_t)ctx->sm_count * 16));
 }
@@ -354,7 +365,8 @@ int tc_gen_parts_lp(tc_ctx *ctx, const tc_ugraph *ug, int k, uint64_t seed, int 
     TC_TRY(batch.alloc(kBatch + 1, s));
     const int32_t cap = (int32_t)std::min<int64_t>(INT32_MAX, (n * 103 + 100LL * k - 1) / (100LL * k));
     const int gv = pgrid(n, ctx);
-    const int gc = (int)std::min<int64_t>((n + kPT - 1) / kPT, (int64_t)ctx->sm_count * 64);
+    const int pw = lp_per_warp(n, k, ctx), per_block = pw * (kPT / 32);
+    const int gc = (int)std::min<int64_t>((n + per_block - 1) / per_block, (int64_t)ctx->sm_count * 64);
     TC_CUDA(cudaMemsetAsync(batch.p, 0, sizeof(LpIter) * (kBatch + 1), s));
     lp_init_kernel<<<gv, kPT, 0, s>>>(la.p, n, k, batch.p[0].size);
     TC_CUDA(cudaGetLastError());
@@ -370,11 +382,14 @@ int tc_gen_parts_lp(tc_ctx *ctx, const tc_ugraph *ug, int k, uint64_t seed, int 
         for (int i = 0; i < m; ++i) {
             const int it = it0 + i;
             if (k <= 8)
-                lp_choose_kernel<1><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, seed, it, i, batch.p, desired.p);
+                lp_choose_kernel<1><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                                                    desired.p);
             else if (k <= 16)
-                lp_choose_kernel<2><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, seed, it, i, batch.p, desired.p);
+                lp_choose_kernel<2><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                                                    desired.p);
             else
-                lp_choose_kernel<0><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, seed, it, i, batch.p, desired.p);
+                lp_choose_kernel<0><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                                                    desired.p);
             lp_migrate_kernel<<<gv, kPT, 0, s>>>(from, desired.p, n, k, cap, seed, it, i, batch.p, to);
             TC_CUDA(cudaGetLastError());
             std::swap(from, to);
