@@ -144,3 +144,39 @@ def test_half_a_million_vertices_every_time(ctx, k):
                 ctx.count(busy)
                 ctx.count_per_root(busy)
             assert np.array_equal(ctx.parts_lp(again, k, seed=seed), want)
+
+
+@pytest.mark.parametrize("k", [2, 8, 9, 16, 17, 64])
+def test_long_rows_that_lie_together(ctx, k):
+    """Ids in order of degree: rows around the lists' borders (64, 255 and 1024
+    neighbours) next to one another; iterations around the first look (two)."""
+    src, dst = gen.chung_lu(30_000, 24.0, seed=3)
+    deg = np.bincount(np.concatenate((src, dst)), minlength=30_000)
+    to = np.empty(30_000, np.int64)
+    to[np.argsort(-deg, kind="stable")] = np.arange(30_000)
+    extra = [(200 + i, 25_000 + j) for i, d in enumerate((64, 65, 255, 256, 1024, 1025, 2100)) for j in range(d)]
+    rp, col = oracle.clean(np.concatenate((to[src], [e[0] for e in extra])), np.concatenate((to[dst], [e[1] for e in extra])))
+    assert (np.diff(rp) > 1024).sum() > 5 and (np.diff(rp) > 255).sum() > 100
+    ug = ctx.upload_ugraph(rp, col)
+    for iterations in (1, 2, 3, 10, 11, 20):
+        got = ctx.parts_lp(ug, k, seed=5, iterations=iterations)
+        assert np.array_equal(got, lp_reference(rp, col, k, 5, iterations))
+
+
+def test_ids_in_order_of_degree_cost_no_more(ctx):
+    """R-MAT 18's long rows were left to a few warps: 2.2 ms where shuffled ids took 0.9."""
+    import time
+    src, dst = gen.rmat(18)
+    deg = np.bincount(np.concatenate((src, dst)), minlength=1 << 18)
+    to = np.empty(1 << 18, np.int64)
+    to[np.argsort(-deg, kind="stable")] = np.arange(1 << 18)
+    best = []
+    for u, v in ((src, dst), (to[src], to[dst])):
+        ug = ctx.ugraph_from_edges(u, v)
+        t = []
+        for _ in range(12):  # (one iteration: the two graphs do not stop at the same one)
+            a = time.perf_counter()
+            ctx.parts_lp(ug, 8, seed=1, iterations=1)
+            t.append(time.perf_counter() - a)
+        best.append(min(t))
+    assert best[1] < 1.5 * best[0]

@@ -246,6 +246,18 @@ inline RowBounds row_bounds(int64_t n_rows, int64_t nnz) {
     return {b < INT32_MAX ? (int32_t)b : INT32_MAX, (int32_t)f};
 }
 #ifdef __CUDACC__
+// Appends x to list, *n entries long, with one atomic for the lanes that are here
+// together (a frontier holds hundreds of thousands of vertices, and one atomic
+// each on the one counter was most of the peeling).
+__device__ __forceinline__ void push_together(int32_t *list, int32_t *n, int32_t x) {
+    const unsigned here = __activemask();
+    const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
+    int at = 0;
+    if (lane == first) at = atomicAdd(n, __popc(here));
+    at = __shfl_sync(here, at, first);
+    list[at + __popc(here & ((1u << lane) - 1u))] = x;
+}
+
 // One thread's rows, then a warp's added to the launch's (all lanes call add).
 struct RowTally {
     int longest = 0;

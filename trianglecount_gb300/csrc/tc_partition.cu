@@ -31,6 +31,8 @@ namespace {
 
 constexpr int kMaxParts = 64;
 constexpr int kPT = 256;  // threads per block
+constexpr int kLpFlight = 4;  // neighbours per lane and round (two: 1.37 instead of 1.31 ms)
+constexpr int kGroupDeg = 255, kAloneDeg = 64, kWarpDeg = 1024;  // see lp_choose_kernel
 constexpr unsigned kFull = 0xffffffffu;
 
 // splitmix64 finaliser (Steele, Lea, Flood, "Fast splittable pseudorandom
@@ -46,17 +48,28 @@ __device__ __forceinline__ uint32_t hash_vl(uint64_t seed, int it, int64_t v, in
     return (uint32_t)(mix64(seed ^ mix64(((uint64_t)it << 40) ^ ((uint64_t)v << 8) ^ (uint64_t)l)) >> 32);
 }
 
+// The vertices of long rows, listed once: a warp takes one of mid at a time and a
+// block one of big, each spread over the whole grid, so that long rows that lie
+// together (ids in order of degree) are not one warp's work.
+struct LpLong {
+    int32_t *mid, *big;
+    int32_t *n;  // vertices in mid, in big
+};
+
 // Labels and wishes are bytes on the device (at most 64 parts): the choose
 // pass gathers one label per neighbour, and 4 x smaller arrays hit closer
 // caches.
-__global__ void lp_init_kernel(uint8_t *label, int64_t n, int k, int32_t *size) {
+__global__ void lp_init_kernel(uint8_t *label, const int32_t *__restrict__ rp, int64_t n, int k, int32_t *size,
+                               int mid_deg, LpLong rows) {
     __shared__ int32_t s[kMaxParts];
     for (int i = threadIdx.x; i < k; i += blockDim.x) s[i] = 0;
     __syncthreads();
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        const int l = (int)(v * k / n);
+        const int l = (int)(v * k / n), d = rp[v + 1] - rp[v];
         label[v] = (uint8_t)l;
         atomicAdd(&s[l], 1);
+        if (d > kWarpDeg) push_together(rows.big, rows.n + 1, (int32_t)v);
+        else if (d > mid_deg) push_together(rows.mid, rows.n, (int32_t)v);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < k; i += blockDim.x)
@@ -103,51 +116,116 @@ __device__ __forceinline__ int lp_pick(const int32_t *h, int k, uint64_t seed, i
     return __shfl_sync(kFull, bl, __ffs(__ballot_sync(kFull, bl >= 0)) - 1);
 }
 
-// Per vertex, the label most common among its neighbours.  A block takes eight
-// times per_warp consecutive vertices, a warp per_warp of them: 32, or fewer while
-// that many would leave SMs without a block (lp_per_warp).  With at most 16 parts, vertices of
-// degree <= 255 (kGroupDeg) are counted by eight lanes each, four at a time:
-// the counts are bytes packed in kWords 64-bit registers per lane and are
+// Per vertex, the label most common among its neighbours.  With at most 16 parts,
+// vertices of degree <= 255 (kGroupDeg) are counted by eight lanes each, four at a
+// time: the counts are bytes packed in kWords 64-bit registers per lane and are
 // summed over the lanes with shuffles -- no histogram in memory, and the warp
 // waits for four vertices' gathers at once.  (One warp per vertex with a shared
 // histogram left most lanes idle on most rows: Chung-Lu n = 500 K, mean degree
-// 16, k = 8, 20 iterations 4.00 ms the whole call, 1.31 ms so.)  Degrees up
-// to kWarpDeg: the warp, its histogram in shared memory; larger ones: the whole
-// block, so that a hub's row is not one warp's chain of gathers.
-constexpr int kLpFlight = 4;  // neighbours per lane and round (two: 1.37 instead of 1.31 ms)
-constexpr int kGroupDeg = 255, kWarpDeg = 1024;
+// 16, k = 8, 20 iterations 4.00 ms the whole call, 1.31 ms so.)  With more parts
+// vertices of degree <= 64 (kAloneDeg) are counted one at a time in the warp's
+// histogram.  A warp takes per_warp consecutive vertices of these: 32, or fewer
+// while that many would leave SMs without a block (lp_per_warp).  The others come
+// from the lists (LpLong): up to degree kWarpDeg a warp each, larger ones the whole
+// block, so that a hub's row is not one warp's chain of gathers.  (With each left
+// to the warp or block that its neighbours in id belong to, graphs whose ids go by degree took
+// 3 to 5 x a warp per vertex: R-MAT 20, k = 8, 7.9 instead of 1.5 ms.)
+// Counts the labels of the row [a, a + d) into h, `step` lanes (or threads) of rank
+// `at` together, four gathers in flight each.
+__device__ __forceinline__ void lp_tally(const int32_t *__restrict__ col, const uint8_t *__restrict__ label, int a, int d,
+                                         int at, int step, int32_t *h) {
+    for (int j = at; j < d; j += 4 * step) {
+        int p[4], q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = j + step * i < d ? __ldg(col + a + j + step * i) : -1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = p[i] >= 0 ? __ldg(label + p[i]) : -1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (q[i] >= 0) atomicAdd(&h[q[i]], 1);
+    }
+}
+
 template <int kWords>
 __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                         const uint8_t *__restrict__ label, int64_t n, int k,
-                                                        int per_warp, uint64_t seed, int it, int i_batch,
+                                                        int per_warp, LpLong rows, uint64_t seed, int it, int i_batch,
                                                         LpIter *batch, int8_t *__restrict__ desired) {
+    constexpr int kMidDeg = kWords > 0 ? kGroupDeg : kAloneDeg;
     __shared__ int32_t hist[kPT / 32][kMaxParts];
     __shared__ int32_t s_flow[kMaxParts * kMaxParts];  // candidates from part a to part b at [a * k + b]
-    __shared__ int s_big[kPT], s_nbig;
     if (lp_stopped(batch, i_batch, n)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < k * k; i += blockDim.x) s_flow[i] = 0;
-    if (threadIdx.x == 0) s_nbig = 0;
     __syncthreads();
     int32_t *h = hist[warp];
-    const int per_block = per_warp * (kPT / 32), slot = warp * per_warp + lane;  // slot: a lane's vertex in its block
+    const int n_mid = rows.n[0], n_big = rows.n[1];
+    // one warp: its finished histogram's pick for vertex v
+    auto decide = [&](const int32_t *counts, int64_t v, int cl) {
+        const int pick = lp_pick(counts, k, seed, it, v, cl, lane);
+        if (lane == 0) {
+            desired[v] = (int8_t)pick;
+            if (pick >= 0) atomicAdd(&s_flow[cl * k + pick], 1);
+        }
+    };
+    for (int b = blockIdx.x; b < n_big; b += gridDim.x) {
+        const int64_t v = rows.big[b];
+        for (int i = lane; i < k; i += 32) h[i] = 0;
+        __syncwarp();
+        const int a = rp[v];
+        lp_tally(col, label, a, rp[v + 1] - a, threadIdx.x, kPT, h);
+        __syncthreads();
+        if (warp == 0) {
+            for (int i = lane; i < k; i += 32) {
+                int t = 0;
+#pragma unroll
+                for (int w = 0; w < kPT / 32; ++w) t += hist[w][i];
+                hist[0][i] = t;
+            }
+            __syncwarp();
+            decide(hist[0], v, label[v]);
+        }
+        __syncthreads();
+    }
+    auto alone = [&](int64_t v, int a, int d, int cl) {  // one vertex by the whole warp
+        for (int i = lane; i < k; i += 32) h[i] = 0;
+        __syncwarp();
+        lp_tally(col, label, a, d, lane, 32, h);
+        __syncwarp();
+        decide(h, v, cl);
+        __syncwarp();
+    };
+    for (int b = blockIdx.x + gridDim.x * warp; b < n_mid; b += gridDim.x * (kPT / 32)) {
+        const int64_t v = rows.mid[b];
+        const int a = rp[v];
+        alone(v, a, rp[v + 1] - a, label[v]);
+    }
+    const int per_block = per_warp * (kPT / 32);
     for (int64_t v0 = (int64_t)blockIdx.x * per_block; v0 < n; v0 += (int64_t)gridDim.x * per_block) {
         const int64_t first = v0 + warp * per_warp, mine = first + lane;
-        const bool has = lane < per_warp && mine < n;
         int rs = 0, d = 0, cur = 0;
+        bool has = lane < per_warp && mine < n;
         if (has) {
             rs = rp[mine];
             d = rp[mine + 1] - rs;
             cur = label[mine];
+            has = d <= kMidDeg;  // the others are listed
         }
-        const bool grouped = kWords > 0 && d <= kGroupDeg;
-        int choice = -1;  // of this lane's vertex
-        if (kWords > 0) {
+        const int mine_d = has ? d : 0;
+        if (kWords == 0) {
+            if (has && d == 0) desired[mine] = -1;
+            for (unsigned todo = __ballot_sync(kFull, mine_d > 0); todo; todo &= todo - 1u) {
+                const int src = __ffs(todo) - 1;
+                alone(first + src, __shfl_sync(kFull, rs, src), __shfl_sync(kFull, mine_d, src),
+                      __shfl_sync(kFull, cur, src));
+            }
+        } else {
+            int choice = -1;  // of this lane's vertex
             const int g = lane >> 3, l8 = lane & 7;
             for (int r = 0; r < per_warp; r += 4) {
                 const int src = r + g;  // the group's vertex: lane src's
                 const int a = __shfl_sync(kFull, rs, src);
-                const int dd = __shfl_sync(kFull, grouped ? d : 0, src), cl = __shfl_sync(kFull, cur, src);
+                const int dd = __shfl_sync(kFull, mine_d, src), cl = __shfl_sync(kFull, cur, src);
                 unsigned long long c[kWords > 0 ? kWords : 1];
 #pragma unroll
                 for (int w = 0; w < kWords; ++w) c[w] = 0;
@@ -200,71 +278,15 @@ __global__ void __launch_bounds__(kPT) lp_choose_kernel(const int32_t *__restric
                 }
                 // lanes r .. r + 3 own the four vertices: group g's pick
                 const int got = __shfl_sync(kFull, pick, ((lane - r) & 3) << 3);
-                if (grouped && lane >= r && lane < r + 4) choice = got;
+                if (lane >= r && lane < r + 4) choice = got;
+            }
+            if (has) {
+                desired[mine] = (int8_t)choice;
+                if (choice >= 0) atomicAdd(&s_flow[cur * k + choice], 1);
             }
         }
-        for (unsigned todo = __ballot_sync(kFull, !grouped && d > 0 && d <= kWarpDeg); todo; todo &= todo - 1u) {
-            const int src = __ffs(todo) - 1;
-            const int a = __shfl_sync(kFull, rs, src), dd = __shfl_sync(kFull, d, src), cl = __shfl_sync(kFull, cur, src);
-            for (int i = lane; i < k; i += 32) h[i] = 0;
-            __syncwarp();
-            for (int j = lane; j < dd; j += 128) {
-                int p[4], q[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) p[i] = j + 32 * i < dd ? __ldg(col + a + j + 32 * i) : -1;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) q[i] = p[i] >= 0 ? __ldg(label + p[i]) : -1;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (q[i] >= 0) atomicAdd(&h[q[i]], 1);
-            }
-            __syncwarp();
-            const int pick = lp_pick(h, k, seed, it, first + src, cl, lane);
-            if (lane == src) choice = pick;
-            __syncwarp();
-        }
-        if (d > kWarpDeg && !grouped) s_big[atomicAdd(&s_nbig, 1)] = slot;
-        __syncthreads();
-        const int nbig = s_nbig;
-        for (int b = 0; b < nbig; ++b) {
-            const int64_t v = v0 + s_big[b];
-            const int a = rp[v], dd = rp[v + 1] - a, cl = label[v];
-            for (int i = lane; i < k; i += 32) h[i] = 0;
-            __syncwarp();
-            for (int j = threadIdx.x; j < dd; j += 4 * kPT) {
-                int p[4], q[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) p[i] = j + kPT * i < dd ? __ldg(col + a + j + kPT * i) : -1;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) q[i] = p[i] >= 0 ? __ldg(label + p[i]) : -1;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (q[i] >= 0) atomicAdd(&h[q[i]], 1);
-            }
-            __syncthreads();
-            if (warp == 0) {
-                for (int i = lane; i < k; i += 32) {
-                    int t = 0;
-#pragma unroll
-                    for (int w = 0; w < kPT / 32; ++w) t += hist[w][i];
-                    hist[0][i] = t;
-                }
-                __syncwarp();
-                const int pick = lp_pick(hist[0], k, seed, it, v, cl, lane);
-                if (lane == 0) {
-                    desired[v] = (int8_t)pick;
-                    if (pick >= 0) atomicAdd(&s_flow[cl * k + pick], 1);
-                }
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) s_nbig = 0;  // read by all before the last barrier above, or none was listed
-        if (has && (grouped || d <= kWarpDeg)) {
-            desired[mine] = (int8_t)choice;
-            if (choice >= 0) atomicAdd(&s_flow[cur * k + choice], 1);
-        }
-        __syncthreads();
     }
+    __syncthreads();
     int32_t *flow = batch[i_batch].flow;
     for (int i = threadIdx.x; i < k * k; i += blockDim.x)
         if (s_flow[i]) atomicAdd(&flow[i], s_flow[i]);
@@ -356,39 +378,42 @@ int tc_gen_parts_lp(tc_ctx *ctx, const tc_ugraph *ug, int k, uint64_t seed, int 
     constexpr int kBatch = 8;  // iterations enqueued per look at the moves
     DBuf<uint8_t> la, lb;
     DBuf<int8_t> desired;
-    DBuf<int32_t> wide;
-    DBuf<LpIter> batch;  // the last one holds the next batch's first sizes
+    DBuf<int32_t> wide, lists;
+    DBuf<LpIter> batch;  // the one after a batch's last holds the next batch's first sizes; behind all, the lists' lengths
     TC_TRY(la.alloc((size_t)n, s));
     TC_TRY(lb.alloc((size_t)n, s));
     TC_TRY(desired.alloc((size_t)n, s));
     TC_TRY(wide.alloc((size_t)n, s));
-    TC_TRY(batch.alloc(kBatch + 1, s));
+    TC_TRY(batch.alloc(kBatch + 2, s));
+    const int mid_deg = k <= 16 ? kGroupDeg : kAloneDeg;
+    const size_t most_mid = (size_t)(ug->nnz / (mid_deg + 1)), most_big = (size_t)(ug->nnz / (kWarpDeg + 1));
+    TC_TRY(lists.alloc(most_mid + most_big, s));
+    const LpLong rows{lists.p, lists.p + most_mid, batch.p[kBatch + 1].size};
     const int32_t cap = (int32_t)std::min<int64_t>(INT32_MAX, (n * 103 + 100LL * k - 1) / (100LL * k));
     const int gv = pgrid(n, ctx);
     const int pw = lp_per_warp(n, k, ctx), per_block = pw * (kPT / 32);
     const int gc = (int)std::min<int64_t>((n + per_block - 1) / per_block, (int64_t)ctx->sm_count * 64);
-    TC_CUDA(cudaMemsetAsync(batch.p, 0, sizeof(LpIter) * (kBatch + 1), s));
-    lp_init_kernel<<<gv, kPT, 0, s>>>(la.p, n, k, batch.p[0].size);
+    TC_CUDA(cudaMemsetAsync(batch.p, 0, sizeof(LpIter) * (kBatch + 2), s));
+    lp_init_kernel<<<gv, kPT, 0, s>>>(la.p, ug->rp, n, k, batch.p[0].size, mid_deg, rows);
     TC_CUDA(cudaGetLastError());
     bool more = k > 1;
-    for (int it0 = 0; it0 < iterations && more; it0 += kBatch) {
-        const int m = std::min(kBatch, iterations - it0);
-        if (it0 > 0) {
-            TC_CUDA(cudaMemcpyAsync(batch.p[0].size, batch.p[kBatch].size, sizeof(LpIter().size),
-                                    cudaMemcpyDeviceToDevice, s));
+    for (int it0 = 0, m = 0; it0 < iterations && more; it0 += m) {
+        if (it0 > 0) {  // the last batch's end is this one's start
+            TC_CUDA(cudaMemcpyAsync(batch.p[0].size, batch.p[m].size, sizeof(LpIter().size), cudaMemcpyDeviceToDevice, s));
             TC_CUDA(cudaMemsetAsync(batch.p[0].flow, 0, sizeof(LpIter) * (kBatch + 1) - sizeof(LpIter().size), s));
         }
+        m = std::min(kBatch, iterations - it0);
         uint8_t *from = la.p, *to = lb.p;
         for (int i = 0; i < m; ++i) {
             const int it = it0 + i;
             if (k <= 8)
-                lp_choose_kernel<1><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                lp_choose_kernel<1><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, rows, seed, it, i, batch.p,
                                                     desired.p);
             else if (k <= 16)
-                lp_choose_kernel<2><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                lp_choose_kernel<2><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, rows, seed, it, i, batch.p,
                                                     desired.p);
             else
-                lp_choose_kernel<0><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, seed, it, i, batch.p,
+                lp_choose_kernel<0><<<gc, kPT, 0, s>>>(ug->rp, ug->col, from, n, k, pw, rows, seed, it, i, batch.p,
                                                     desired.p);
             lp_migrate_kernel<<<gv, kPT, 0, s>>>(from, desired.p, n, k, cap, seed, it, i, batch.p, to);
             TC_CUDA(cudaGetLastError());

@@ -489,18 +489,6 @@ __device__ __forceinline__ int halo_rank(int a, unsigned long long rk, const int
     return off[c * tiles + t] - off[c * tiles] + (int)((rk >> (c * kRankBits)) & kRankMask);
 }
 
-// Appends x to list, *n entries long, with one atomic for the lanes that are here
-// together (a frontier holds hundreds of thousands of vertices, and one atomic
-// each on the one counter was most of the peeling).
-__device__ __forceinline__ void push_together(int32_t *list, int32_t *n, int32_t x) {
-    const unsigned here = __activemask();
-    const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
-    int at = 0;
-    if (lane == first) at = atomicAdd(n, __popc(here));
-    at = __shfl_sync(here, at, first);
-    list[at + __popc(here & ((1u << lane) - 1u))] = x;
-}
-
 // Per vertex of the part's combined set: its P and H entry counts (from the
 // ranks at its row's start and at the next row's start), the bases that turn an
 // entry's global rank into its local-row offset, and the in-degree of a halo
