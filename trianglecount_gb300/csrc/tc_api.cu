@@ -186,8 +186,11 @@ int ensure_count_scratch(tc_graph *g) {
     if (!g->d_desc) {  // the flat count needs only the work words
         TC_TRY(dalloc((void **)&g->d_desc, sizeof(GraphDesc), ctx->stream));
     }
-    TC_TRY(scratch_alloc(&g->sc, g->n_rows + 1, g->nnz, std::min(g->n_rows, g->nnz) + 1, 1, packed_graph(g),
-                         ctx->stream));
+    const bool want = packed_graph(g);
+    bool packed = want;
+    TC_TRY(scratch_alloc_either(&g->sc, g->n_rows + 1, g->nnz, std::min(g->n_rows, g->nnz) + 1, 1, &packed,
+                                ctx->stream));
+    if (want && !packed) g->no_pack = true;  // from now on, so that no count tries again
     return TC_OK;
 }
 
@@ -291,7 +294,7 @@ bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     }
     return 2 * gain >= E && kFarShare * far <= E && of_roots >= E / 16 + V / 4 && pack_fits(V, E);
 }
-bool packed_graph(const tc_graph *g) { return packed_graphs(&g, 1, g->ctx->tuned); }
+bool packed_graph(const tc_graph *g) { return !g->no_pack && packed_graphs(&g, 1, g->ctx->tuned); }
 
 // A wrapped graph's arrays are the caller's, and only a count may read them: the
 // first one that waits for its result anyway also looks at the rows.  They decide
@@ -461,6 +464,7 @@ int dalloc(void **p, size_t bytes, cudaStream_t s) {
     cudaError_t e = cudaMallocAsync(p, bytes, s);
     if (e != cudaSuccess) {
         *p = nullptr;
+        cudaGetLastError();  // the caller may go on with less; launches that follow are not to see it
         return cuda_error(e, "cudaMallocAsync", __FILE__, __LINE__);
     }
     return TC_OK;
@@ -512,6 +516,14 @@ int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int
     TC_TRY(dalloc((void **)&sc->in_list, sizeof(int32_t) * (size_t)std::max<int64_t>(E, 1), s));
     TC_TRY(dalloc((void **)&sc->mid, (size_t)std::max<int64_t>(E, 1), s));
     return TC_OK;
+}
+
+int scratch_alloc_either(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool *packed,
+                         cudaStream_t s) {
+    const int st = scratch_alloc(sc, V, E, heavy_cap, n_graphs, *packed, s);
+    if (st != TC_E_NOMEM || !*packed) return st;
+    *packed = false;
+    return scratch_alloc(sc, V, E, heavy_cap, n_graphs, false, s);
 }
 
 void scratch_free(CountScratch *sc, cudaStream_t s) {
@@ -577,7 +589,7 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
-    const bool packed = packed_graphs(graphs, n, ctx->tuned);
+    bool packed = packed_graphs(graphs, n, ctx->tuned);
     CountScratch sc;
     DBuf<GraphDesc> d_desc;
     DBuf<unsigned char> d_work;
@@ -592,7 +604,7 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
     }
     int st = d_desc.alloc((size_t)n, s);
     if (st == TC_OK) st = d_work.alloc(out_bytes, s);
-    if (st == TC_OK) st = scratch_alloc(&sc, vtot, etot, cap, n, packed, s);
+    if (st == TC_OK) st = scratch_alloc_either(&sc, vtot, etot, cap, n, &packed, s);
     if (st == TC_OK && cudaMemcpyAsync(d_desc.p, desc.data(), sizeof(GraphDesc) * (size_t)n, cudaMemcpyHostToDevice,
                                        s) != cudaSuccess)
         st = set_error(TC_E_CUDA, "descriptor upload failed");
@@ -1098,11 +1110,11 @@ int tc_batch_create(tc_ctx *ctx, tc_graph *const *graphs, int n, tc_batch **out)
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
-    const bool packed = packed_graphs(graphs, n, ctx->tuned);
+    bool packed = packed_graphs(graphs, n, ctx->tuned);
     b->total_chunks = chunks;
     b->total_vertices = vtot;
     int st = dalloc((void **)&b->d_desc, sizeof(GraphDesc) * (size_t)n, s);
-    if (st == TC_OK) st = scratch_alloc(&b->sc, vtot, etot, cap, n, packed, s);
+    if (st == TC_OK) st = scratch_alloc_either(&b->sc, vtot, etot, cap, n, &packed, s);
     if (st == TC_OK) st = dalloc((void **)&b->d_work, sizeof(CountWork) + sizeof(unsigned long long) * (size_t)n, s);
     if (st == TC_OK && cudaMallocHost(&b->h_out, sizeof(CountWork) + sizeof(unsigned long long) * (size_t)n) != cudaSuccess)
         st = set_error(TC_E_NOMEM, "pinned result buffer");
@@ -1196,11 +1208,11 @@ int enqueue_group_count(tc_ctx *ctx, tc_graph *const *gs, int n, unsigned long l
         etot += g->nnz;
         cap += std::min(g->n_rows, g->nnz) + 1;
     }
-    const bool packed = packed_graphs(gs, n, ctx->tuned);
+    bool packed = packed_graphs(gs, n, ctx->tuned);
     grp->s = s;
     TC_TRY(grp->desc.alloc((size_t)n, s));
     TC_TRY(grp->work.alloc(1, s));
-    TC_TRY(scratch_alloc(&grp->sc, vtot, etot, cap, n, packed, s));
+    TC_TRY(scratch_alloc_either(&grp->sc, vtot, etot, cap, n, &packed, s));
     for (int i0 = 0; i0 < n; i0 += 8) {
         DescBlock blk;
         const int m = std::min(8, n - i0);

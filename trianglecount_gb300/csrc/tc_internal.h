@@ -108,6 +108,10 @@ struct CountScratch {
 // Allocates the arrays of the packed or the plain-id count, where sc does not have them yet.
 int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool packed,
                   cudaStream_t s);
+// The same, the plain-id count's (less per row) where the packed count's do not fit
+// the memory; *packed then says so.
+int scratch_alloc_either(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool *packed,
+                         cudaStream_t s);
 void scratch_free(CountScratch *sc, cudaStream_t s);
 
 // Per-launch device words, zeroed by one memset before each count.
@@ -328,6 +332,7 @@ struct tc_graph {
     int64_t root_nnz = -1; // entries in the roots' rows; -1: not known
     bool owns = true;
     bool loop_free = false;  // no row holds its own id (device-built graphs)
+    bool no_pack = false;    // the packed count's scratch did not fit the memory
     // per-graph count scratch, sized on first use
     tc::GraphDesc *d_desc = nullptr;
     tc::CountWork *d_work = nullptr;
