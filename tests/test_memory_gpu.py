@@ -87,3 +87,25 @@ def test_a_count_that_does_not_fit_packed_counts_on_plain_ids(own):
         own.synchronize()
     assert own.count(g, stats=True)[1]["launches"] == 5 and own.count(g) == want
     g.free()
+
+
+def test_a_count_that_does_not_fit_at_all_leaves_nothing_behind(own):
+    rp, col, want = oracle.pipeline(*gen.rmat(16))
+    rp = among(rp, 2_000_000)
+    own.set_tuning(probe_kicks=0)  # the plain-id tables
+    g = own.upload(rp, col)
+    with Pool(32 * MB) as pool:
+        used = []
+        for _ in range(4):
+            with pytest.raises(tc.TCError) as e:
+                own.count(g)
+            assert e.value.code == "TC_E_NOMEM"
+            own.synchronize()
+            used.append(pool.get(Pool.USED))
+        assert max(used) < MB
+        kept = own.upload(np.array([0, 2, 3, 3], np.int32), np.array([1, 2, 2], np.int32))
+        assert own.count(kept) == 1
+        kept.free()
+        own.synchronize()
+    assert own.count(g) == want
+    g.free()

@@ -496,6 +496,21 @@ void ctx_release(tc_ctx *c) {
     delete c;
 }
 
+// The plain-id count's arrays; the packed count's stay.
+static void plain_scratch_free(CountScratch *sc, cudaStream_t s) {
+    dfree(sc->heavy, s);
+    dfree(sc->light_list, s);
+    dfree(sc->in_cnt, s);
+    dfree(sc->in_off, s);
+    dfree(sc->in_work, s);
+    dfree(sc->out_work, s);
+    dfree(sc->in_list, s);
+    dfree(sc->mid, s);
+    const PackScratch pk = sc->pk;
+    *sc = CountScratch();
+    sc->pk = pk;
+}
+
 int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool packed,
                   cudaStream_t s) {
     // in-list offsets and slots are int32 over the launch's pooled edges
@@ -506,16 +521,18 @@ int scratch_alloc(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int
                          (long long)E);
     if (packed) return sc->pk.units ? TC_OK : pack_scratch_alloc(&sc->pk, V, E, n_graphs, s);
     if (sc->mid) return TC_OK;
+    const size_t v = (size_t)std::max<int64_t>(V, 1), e = (size_t)std::max<int64_t>(E, 1);
     sc->heavy_cap = heavy_cap;
-    TC_TRY(dalloc((void **)&sc->heavy, sizeof(HeavyEntry) * (size_t)std::max<int64_t>(heavy_cap, 1), s));
-    TC_TRY(dalloc((void **)&sc->light_list, sizeof(uint32_t) * (size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(dalloc((void **)&sc->in_cnt, sizeof(int32_t) * (size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(dalloc((void **)&sc->in_off, sizeof(int32_t) * (size_t)(V + 1), s));
-    TC_TRY(dalloc((void **)&sc->in_work, sizeof(unsigned long long) * (size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(dalloc((void **)&sc->out_work, sizeof(unsigned long long) * (size_t)std::max<int64_t>(V, 1), s));
-    TC_TRY(dalloc((void **)&sc->in_list, sizeof(int32_t) * (size_t)std::max<int64_t>(E, 1), s));
-    TC_TRY(dalloc((void **)&sc->mid, (size_t)std::max<int64_t>(E, 1), s));
-    return TC_OK;
+    int st = dalloc((void **)&sc->heavy, sizeof(HeavyEntry) * (size_t)std::max<int64_t>(heavy_cap, 1), s);
+    if (st == TC_OK) st = dalloc((void **)&sc->light_list, sizeof(uint32_t) * v, s);
+    if (st == TC_OK) st = dalloc((void **)&sc->in_cnt, sizeof(int32_t) * v, s);
+    if (st == TC_OK) st = dalloc((void **)&sc->in_off, sizeof(int32_t) * (size_t)(V + 1), s);
+    if (st == TC_OK) st = dalloc((void **)&sc->in_work, sizeof(unsigned long long) * v, s);
+    if (st == TC_OK) st = dalloc((void **)&sc->out_work, sizeof(unsigned long long) * v, s);
+    if (st == TC_OK) st = dalloc((void **)&sc->in_list, sizeof(int32_t) * e, s);
+    if (st == TC_OK) st = dalloc((void **)&sc->mid, e, s);  // the last: its presence says that all are there
+    if (st != TC_OK) plain_scratch_free(sc, s);
+    return st;
 }
 
 int scratch_alloc_either(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_cap, int n_graphs, bool *packed,
@@ -527,14 +544,7 @@ int scratch_alloc_either(CountScratch *sc, int64_t V, int64_t E, int64_t heavy_c
 }
 
 void scratch_free(CountScratch *sc, cudaStream_t s) {
-    dfree(sc->heavy, s);
-    dfree(sc->light_list, s);
-    dfree(sc->in_cnt, s);
-    dfree(sc->in_off, s);
-    dfree(sc->in_work, s);
-    dfree(sc->out_work, s);
-    dfree(sc->in_list, s);
-    dfree(sc->mid, s);
+    plain_scratch_free(sc, s);
     pack_scratch_free(&sc->pk, s);
     *sc = CountScratch();
 }
