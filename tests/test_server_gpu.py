@@ -169,3 +169,19 @@ def test_one_key_built_by_both_lanes_at_once(ctx):
             assert srv.wait(srv.submit(key=99))[0] == want
         st = srv.stats()
     assert st["failed"] == 0 and st["resident_graphs"] == 1
+
+
+def test_budget_charges_a_graph_by_the_count_it_takes(ctx):
+    """Four road grids of a million vertices fit at 64 MB each (the CSR and the
+    plain-id tables), not at the 91 MB that the packed count would take."""
+    side = 1024
+    gs = [gen.road(side, seed=s) for s in range(4)]
+    want = [ctx.count(ctx.graph_from_edges(s, d)) for s, d in gs]
+    build = 58 * max(len(s) for s, _ in gs) + (1 << 20)
+    with tc.Server(ctx, hbm_budget_bytes=3 * (72 << 20) + build + (8 << 20)) as srv:
+        for k, (s, d) in enumerate(gs):
+            assert srv.wait(srv.submit(s, d, key=k + 1))[0] == want[k]
+        for k in range(4):
+            assert srv.wait(srv.submit(key=k + 1))[0] == want[k]
+        st = srv.stats()
+    assert st["evictions"] == 0 and st["cache_hits"] == 4 and st["used_bytes"] <= st["budget_bytes"]

@@ -567,10 +567,12 @@ int graph_rebind(tc_graph *g, tc_ctx *ctx) {
 }
 
 size_t graph_device_bytes(const tc_graph *g) {
-    const size_t csr = sizeof(int32_t) * (size_t)(g->n_rows + 1 + g->nnz);
-    // the larger of the two counts' scratch per row (packed: code, place, padding) and per edge
-    const size_t scratch = (size_t)(g->n_rows + 1) * (4 + 16 + 52) + (size_t)g->nnz * 5 + 4096;
-    return csr + scratch;
+    const size_t V = (size_t)g->n_rows + 1, E = (size_t)g->nnz;
+    const size_t plain = V * (4 + 4 + 4 + 8 + 8) + std::min(V, E + 1) * sizeof(HeavyEntry) + E * 5;
+    const size_t packed = pack_scratch_bytes((int64_t)V, (int64_t)E, 1);
+    // what it has, or what its count will take (in a batch, its share of the batch's)
+    const size_t held = (g->sc.mid ? plain : 0) + (g->sc.pk.units ? packed : 0);
+    return sizeof(int32_t) * (V + E) + std::max(held, packed_graph(g) ? packed : plain) + 4096;
 }
 
 int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *outs, int64_t timeout_ms,

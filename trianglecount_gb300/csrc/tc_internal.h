@@ -161,6 +161,7 @@ inline bool packed_count(const Tuned &tn) {
 }
 bool pack_fits(int64_t V, int64_t E);  // else the plain-id tables count it
 int pack_mask_bits(int64_t n_rows);
+size_t pack_scratch_bytes(int64_t V, int64_t E, int n_graphs);
 int pack_scratch_alloc(PackScratch *ps, int64_t V, int64_t E, int n_graphs, cudaStream_t s);
 void pack_scratch_free(PackScratch *ps, cudaStream_t s);
 // The packed count's persistent grid, num / den of what fits (a grid kept below
@@ -293,7 +294,7 @@ int count_graphs_direct(tc_ctx *ctx, tc_graph *const *graphs, int n, uint64_t *o
                         float *kernel_ms);
 // Moves a graph to another context of the same device (reference counts follow).
 int graph_rebind(tc_graph *g, tc_ctx *ctx);
-// Device bytes held by a graph (CSR + count scratch once sized).
+// Device bytes of a graph: its CSR, and the scratch that it has or that its count takes.
 size_t graph_device_bytes(const tc_graph *g);
 
 // Context lifetime: every graph, ugraph and batch holds a reference to its

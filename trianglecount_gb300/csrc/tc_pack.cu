@@ -1129,6 +1129,13 @@ int pack_mask_bits(int64_t n_rows) {
 
 bool pack_fits(int64_t V, int64_t E) { return E + kRowPad * V + 8 < ((int64_t)1 << 34); }  // quads numbered in 32 bits
 
+size_t pack_scratch_bytes(int64_t V, int64_t E, int n_graphs) {
+    const size_t v = (size_t)std::max<int64_t>(V, 1), e = (size_t)std::max<int64_t>(E, 1);
+    return sizeof(uint32_t) * (v + (size_t)n_graphs * 2 * kBuckets) + sizeof(int4) * v +
+           sizeof(uint32_t) * (e + kRowPad * v + 8) + sizeof(uint32_t) * (e / (kRowMax + 1) + 1) +
+           sizeof(uint2) * (e / (kRowMax / 2) + 1);
+}
+
 int pack_scratch_alloc(PackScratch *ps, int64_t V, int64_t E, int n_graphs, cudaStream_t s) {
     const size_t v = (size_t)std::max<int64_t>(V, 1), e = (size_t)std::max<int64_t>(E, 1);
     int st = dalloc((void **)&ps->code, sizeof(uint32_t) * (v + (size_t)n_graphs * 2 * kBuckets), s);

@@ -65,6 +65,7 @@ struct Request {
     uint64_t count = 0;
     tc_graph *g = nullptr;
     bool owns_graph = false;  // graph without a key: freed after the count
+    size_t bytes = 0;         // ... and what the budget was charged for it
 };
 
 struct Resident {
@@ -286,6 +287,7 @@ void prep_loop(tc_server *s, int li) {
             res.lane = li;
         } else {
             r->owns_graph = true;
+            r->bytes = bytes;
         }
         r->state = kReady;
         L.ready.push_back(r);
@@ -329,7 +331,7 @@ void count_loop(tc_server *s, int li) {
             r->count = outs[i];
             finish(s, r, st, st == TC_OK ? nullptr : err.c_str());
             if (r->owns_graph) {
-                s->used -= tc::graph_device_bytes(r->g);
+                s->used -= r->bytes;
                 if (st != TC_E_TIMEOUT) tc_graph_destroy(r->g);
             } else if (r->key) {
                 auto it = s->cache.find(r->key);
