@@ -263,23 +263,37 @@ __device__ __forceinline__ void push_together(int32_t *list, int32_t *n, int32_t
     list[at + __popc(here & ((1u << lane) - 1u))] = x;
 }
 
-// One thread's rows, then a warp's added to the launch's (all lanes call add).
+// One thread's rows, then a block's added to the launch's: all its threads call add,
+// once (one warp's sums at a time were 150 K atomics on one line for every part of a
+// halo extraction, 30 us of its 1 ms).
 struct RowTally {
     int longest = 0;
-    unsigned skewed = 0, far = 0;
+    unsigned skewed = 0, far = 0, of_roots = 0;
     __device__ __forceinline__ void row(int d, RowBounds b) {
         longest = max(longest, d);
         if (d > b.skew) skewed += (unsigned)d;
         if (d > b.far) far += (unsigned)d;
     }
-    __device__ __forceinline__ void add(RowStats *out) {
+    __device__ __forceinline__ void add(RowStats *out, int32_t *root_nnz = nullptr) {
+        __shared__ int s_longest;
+        __shared__ unsigned s_sum[3];
+        if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+        if (threadIdx.x == 0) s_longest = 0;
+        __syncthreads();
         longest = __reduce_max_sync(0xffffffffu, longest);
-        skewed = __reduce_add_sync(0xffffffffu, skewed);
-        far = __reduce_add_sync(0xffffffffu, far);
+        const unsigned sum[3] = {__reduce_add_sync(0xffffffffu, skewed), __reduce_add_sync(0xffffffffu, far),
+                                 __reduce_add_sync(0xffffffffu, of_roots)};
         if ((threadIdx.x & 31) == 0 && longest) {
-            atomicMax(&out->longest, longest);
-            if (skewed) atomicAdd(&out->skewed, skewed);
-            if (far) atomicAdd(&out->far, far);
+            atomicMax(&s_longest, longest);
+            for (int i = 0; i < 3; ++i)
+                if (sum[i]) atomicAdd(&s_sum[i], sum[i]);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && s_longest) {
+            atomicMax(&out->longest, s_longest);
+            if (s_sum[0]) atomicAdd(&out->skewed, s_sum[0]);
+            if (s_sum[1]) atomicAdd(&out->far, s_sum[1]);
+            if (root_nnz && s_sum[2]) atomicAdd(root_nnz, (int)s_sum[2]);
         }
     }
 };

@@ -577,7 +577,6 @@ __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__re
                                 int32_t *__restrict__ lid, int32_t *__restrict__ len, RowBounds bounds, HaloWords *words) {
     const int t_ver = (int)(ids[V] & 0xffffffffll);
     RowTally t;
-    int of_roots = 0;
     GRID_STRIDE(v, V) {
         const int c = cd[v].x;
         int l = -1;
@@ -587,12 +586,10 @@ __global__ void halo_ids_kernel(const int2 *__restrict__ cd, const uint8_t *__re
         if (l >= 0) {
             len[l] = cnt[v];
             t.row(cnt[v], bounds);
-            if (c == 0) of_roots += cnt[v];
+            if (c == 0) t.of_roots += (unsigned)cnt[v];
         }
     }
-    t.add(&words->rows);
-    of_roots = __reduce_add_sync(kFull, of_roots);
-    if ((threadIdx.x & 31) == 0 && of_roots) atomicAdd(&words->root_nnz, of_roots);
+    t.add(&words->rows, &words->root_nnz);
 }
 
 // Pass 2 (strided): ranks each tile's P and H entries again from the stored
