@@ -48,3 +48,23 @@ def test_autotune_respects_budget_ranges_and_counts(fresh, maker, max_trials):
     assert all(cur[k] == tuning[k] for k in RANGES)  # the picked tuning is the context's
     assert fresh.count(g) == want
     assert np.array_equal(fresh.count_per_root(g), want_pr)
+
+
+@pytest.mark.parametrize("maker, most", [("rmat17", 30), ("er_small", 20), ("road", 12), ("er_large", 10**6)])
+def test_autotune_times_no_candidate_that_launches_the_same(fresh, maker, most):
+    """The packed count reads two of the thresholds and the one-kernel counts none:
+    a pass over the grid is 12 trials for the first (24 of every candidate), 8 and
+    1 for the others, and 25 on the plain-id tables."""
+    src, dst = {"rmat17": lambda: gen.rmat(17), "er_small": lambda: gen.er(10_000, 24.0, seed=3),
+                "road": lambda: gen.road(200), "er_large": lambda: gen.er(100_000, 16.0, seed=3)}[maker]()
+    g = fresh.graph_from_edges(src, dst)
+    want = fresh.count(g)
+    default = fresh.get_tuning()
+    tuning, _, trials = fresh.autotune(g, max_trials=200, reps=1, with_trials=True)
+    assert trials <= most
+    if maker in ("rmat17", "er_small") and not any(tuning[k] for k in ("heavy_bitmap", "hash_pairs", "intersect")) \
+            and tuning["probe_kicks"] > 0:  # what the packed count does not read stays as it was
+        assert all(tuning[k] == default[k] for k in ("light_max_work", "long_list"))
+    if maker == "er_large":
+        assert trials >= 20
+    assert fresh.count(g) == want

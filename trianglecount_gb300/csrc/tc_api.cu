@@ -439,6 +439,14 @@ int new_graph(tc_ctx *ctx, int64_t n_rows, int64_t nnz, int64_t n_roots, tc_grap
 
 }  // namespace
 
+CountRoute count_route(const tc_graph *g) {
+    const Tuned &tn = g->ctx->tuned;
+    if (flat_count(g)) return {CountRoute::kFlat, 0, 0};
+    if (single_count(g)) return {CountRoute::kSingle, 0, 0};
+    if (packed_graph(g)) return {CountRoute::kPacked, tn.warp_max, pack_slice(tn)};
+    return {CountRoute::kPlain, 0, 0};
+}
+
 int validate_csr(tc_ctx *ctx, const int32_t *rp, const int32_t *col, int64_t n_rows, int64_t nnz) {
     return validate_csr_impl(ctx, rp, col, n_rows, nnz);
 }

@@ -170,6 +170,20 @@ int pack_blocks(int sm_count, int num, int den, int *out);
 int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, int64_t total_vertices,
                   int64_t total_edges, const PackScratch &ps, CountWork *work, unsigned long long *results,
                   bool per_root, const Tuned &tn, cudaStream_t s, int *launches, cudaEvent_t *kev);
+// Out-neighbours per block unit of the packed count: 32 to 512.
+inline int pack_slice(const Tuned &tn) {
+    const int s = tn.unit_work / 2048;
+    return s < 32 ? 32 : s > 512 ? 512 : s;
+}
+// What a count of g launches under its context's tuning, as far as the tuning decides it.
+struct CountRoute {
+    enum Form { kFlat, kSingle, kPacked, kPlain } form;
+    int warp_max, slice;  // of the packed count
+    bool same(const CountRoute &o) const {  // (the plain-id count reads every threshold)
+        return form == o.form && form != kPlain && warp_max == o.warp_max && slice == o.slice;
+    }
+};
+CountRoute count_route(const tc_graph *g);
 // One-kernel count of a graph of few edges, on its own ids.
 int launch_single(const GraphDesc &d, CountWork *work, unsigned long long *result, const Tuned &tn, cudaStream_t s,
                   int *launches, cudaEvent_t *kev);

@@ -1184,7 +1184,7 @@ int launch_packed(const GraphDesc *d_desc, int n_graphs, int64_t total_chunks, i
         // a warp's millisecond).  Units of 512 out-neighbours (unit_work / 2048): with 128 a row's table was built
         // four times as often (3.37 ms; R-MAT 23's eight parts 32.9, 30.6 with 512).
         P.warp_max = 2 * tn.warp_max;
-        P.slice = std::min(512, std::max(32, tn.unit_work / 2048));
+        P.slice = pack_slice(tn);
         TC_CUDA(cudaMemsetAsync(ps.code, 0,
                                 sizeof(uint32_t) * ((size_t)total_vertices + (size_t)n_graphs * 2 * kBuckets), s));
         const int64_t tiles = (total_edges + kPopTile - 1) / kPopTile;

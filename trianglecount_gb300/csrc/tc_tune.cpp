@@ -1,14 +1,17 @@
 // tc_tune.cpp -- autotuner for the counting kernel's strategy thresholds.
 //
-// The thresholds decide, per vertex task, warp vs block execution
-// (warp_max_deg, light_max_work), the size of block units (unit_work) and,
-// per partner list, whole-warp streaming vs lane flattening (long_list).
+// The thresholds decide, on the plain-id tables, per vertex task warp vs block
+// execution (warp_max_deg, light_max_work), the size of block units (unit_work)
+// and, per partner list, whole-warp streaming vs lane flattening (long_list);
 // probe_kicks picks the hash (cuckoo or linear probing); intersect the
 // bulk-staged sorted lists instead of hash tables, for all tasks or per task.
+// The packed count of skewed graphs reads warp_max_deg and unit_work only, and
+// probe_kicks = 0, heavy_bitmap, hash_pairs and intersect leave it for the tables.
 // Their best values depend on the degree distribution, so they are picked per
 // graph by timing the real count: coordinate descent from the current tuning,
 // one parameter at a time over a small candidate grid, repeated until a pass
-// changes nothing or the trial budget is spent.
+// changes nothing or the trial budget is spent.  A candidate that launches what
+// the current tuning launches is not timed.
 #include <algorithm>
 #include <vector>
 
@@ -49,6 +52,7 @@ extern "C" int tc_autotune_ex(tc_ctx *ctx, tc_graph *g, int max_trials, int reps
     float cur_ms = 0;
     TC_TRY(time_count(ctx, g, reps, &cur_ms));
     int trials = 1;
+    tc::CountRoute route = tc::count_route(g);
     const std::vector<int32_t> grid[9] = {
         {64, 128, 256, 512},
         {4096, 8192, 16384, 32768, 65536, 131072},
@@ -79,12 +83,15 @@ extern "C" int tc_autotune_ex(tc_ctx *ctx, tc_graph *g, int max_trials, int reps
                 if (*field == v) continue;
                 *field = v;
                 TC_TRY(tc_ctx_set_tuning(ctx, &t));
+                const tc::CountRoute to = tc::count_route(g);
+                if (to.same(route)) continue;
                 float ms = 0;
                 TC_TRY(time_count(ctx, g, reps, &ms));
                 ++trials;
                 if (ms < cur_ms * 0.98f) {  // keep a change only if it clearly helps
                     cur = t;
                     cur_ms = ms;
+                    route = to;
                     changed = true;
                 }
             }
