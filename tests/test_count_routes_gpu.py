@@ -262,3 +262,48 @@ def test_a_callers_capture_outlives_the_look_at_the_rows():
         assert int(out.item()) == want and c.count(g) == want
     g.free()
     c.close()
+
+
+@pytest.fixture
+def tuned(ctx):
+    old = ctx.get_tuning()
+    yield ctx
+    ctx.set_tuning(old["warp_max_deg"], old["light_max_work"], old["unit_work"], old["long_list"],
+                   old["probe_kicks"], old["heavy_bitmap"], 0, old["hash_pairs"], old["flat_max_deg"],
+                   old["intersect"])
+
+
+@pytest.mark.parametrize("n", [61_000, 61_440, 61_441, 62_000])
+@pytest.mark.parametrize("deg", [40.0, 100.0])
+def test_unskewed_graphs_on_either_side_of_61440_rows(tuned, n, deg):
+    """Micro, light and heavy tasks of the plain-id cuckoo tables, whole, as a prefix of roots and batched."""
+    rp, col = by_degree(n, *gen.er(n, deg, seed=11))
+    for tuning in ({}, {"warp_max_deg": 32, "unit_work": 64}, {"light_max_work": 16}, {"warp_max_deg": 32, "unit_work": 4096}):
+        tuned.set_tuning(warp_max_deg=256, light_max_work=8192, unit_work=1 << 20)
+        tuned.set_tuning(**tuning)
+        for n_roots in (None, 1000, n // 2):
+            assert (launches_of(tuned, rp, col, n_roots) > PACKED) == (n > 61_440)
+        if n > 61_440 and tuning.get("warp_max_deg") == 32:
+            assert tuned.count(tuned.upload(rp, col), stats=True)[1]["heavy_units"] > 0
+
+
+@pytest.mark.parametrize("more", ["plain", "packed"])
+def test_mixed_batches_go_with_most_of_their_edges(tuned, more):
+    """Unskewed and skewed graphs and halo parts in one launch, on the tables and packed."""
+    er = by_degree(100_000, *gen.er(100_000, 16.0, seed=3))
+    src, dst = gen.rmat(16)
+    skewed = oracle.pipeline(src, dst)[:2]
+    ug = tuned.ugraph_from_edges(src, dst)
+    parts = tuned.halo_extract(ug, gen.parts_random(ug.info()[0], 3), 3, mode="count")
+    plain = [er] * (5 if more == "plain" else 1)
+    graphs = [tuned.upload(*c) for c in plain + [skewed]] + parts
+    want = [oracle.count(*c) for c in plain + [skewed]] + [tuned.count(p) for p in parts]
+    assert sum(want[-3:]) == want[len(plain)]
+    gain = sum(g.nnz for g in graphs) - len(plain) * len(er[1])
+    assert (2 * gain >= sum(g.nnz for g in graphs)) == (more == "packed")
+    for tuning in ({}, {"warp_max_deg": 32, "unit_work": 64}):
+        tuned.set_tuning(**tuning)
+        for order in (1, -1):
+            b = tuned.batch(graphs[::order])
+            assert list(b.run()) == want[::order]
+            assert (b.stats()["launches"] == PACKED) == (more == "packed")
