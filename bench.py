@@ -22,12 +22,11 @@ Printed on rank 0 as ONE JSON line:
   e2e        the same metric through the C ABI (tc_count_parts_csr_i32) from
              pinned host buffers of the k = 8 parts: upload + validation +
              batched count + result read-back
-  roofline   of the dominant kernel (packed_kernel of the batched launch):
-             achieved = the bytes of a count by cheaper sides on plain ids (each
-             root list, each edge's row_ptr pair and the cheaper side's list) / its
-             device time (the kernel itself reads packed entries of every list);
-             the DRAM traffic of one launch (ncu) and the every-wedge byte
-             model (every N+(v) read, the reference's probes) beside it
+  roofline   of the dominant kernel (packed_kernel of the batched launch, named
+             by what ran): achieved = the bytes that it reads (PACKED_BYTES, mostly
+             from L2) / its device time; the DRAM traffic of one launch (ncu) and
+             the every-wedge byte model (every N+(v) read, the reference's probes)
+             beside it
   cpu_baseline  the OpenMP merge-intersection oracle on the machine's host cores,
              one full count of the graph
   reference_gpu_kernel  the reference's own TC_128 kernel (built from its
@@ -257,6 +256,53 @@ def load_traffic(workload: str):
     return out
 
 
+def counting_kernel(launches, longest):
+    """The kernel that counts, by the launches of one count: a flat or single
+    launch; the packed count's five; else the plain-id tables' sequence."""
+    if launches <= 1:
+        return "flat4_kernel" if longest <= 4 else "flat_kernel" if longest <= 8 else "single_kernel"
+    return "packed_kernel" if launches == 5 else "count_kernel"
+
+
+PACKED_BYTES = ("the bytes that packed_kernel reads: per root of two or more members 4 (its id) + 16 (its place) per "
+                "out-neighbour, and the out-neighbour's quads of 16 bytes (octets of low blocks if the root has any, "
+                "quads of high blocks once per tile of the root's own); entries by exact popularity, which the "
+                "launch samples.  Most come from L2: dram_frac is the share of HBM's rate")
+
+
+def packed_bytes(rp, col, n_roots, dev):
+    """PACKED_BYTES of one graph (the layout of csrc/tc_pack.cu restated on the GPU)."""
+    import torch
+    rp = torch.from_numpy(np.ascontiguousarray(rp)).to(dev).long()
+    col = torch.from_numpy(np.ascontiguousarray(col)).to(dev).long()
+    n, of_roots = len(rp) - 1, int(rp[n_roots])
+    if of_roots == 0:
+        return 0
+    low_ids = 2048 * 15
+    mb = 16
+    while mb > 1 and (n + mb - 1) // mb > 31 << (27 - mb):
+        mb -= 1
+    d = rp[1:] - rp[:-1]
+    row = torch.repeat_interleave(torch.arange(n, device=dev), d)
+    rank = torch.empty(n, dtype=torch.int64, device=dev)
+    rank[torch.argsort(torch.bincount(col[:of_roots], minlength=n), descending=True)] = torch.arange(n, device=dev)
+    r = rank[col]
+    low, short = r < low_ids, d[row] <= 32
+
+    def blocks(which, width, per_row):  # different blocks of a row
+        key = torch.unique(row[which] * per_row + torch.div(r[which], width, rounding_mode="floor"))
+        return torch.bincount(torch.div(key, per_row, rounding_mode="floor"), minlength=n)
+
+    n_low = blocks(low, 15, 2048)
+    n_high = blocks(~low & short, mb, n // mb + 1) + torch.bincount(row[~low & ~short], minlength=n)
+    octets, quads = (n_low + 7) // 8, (n_high + 3) // 4
+    tile = torch.where(d <= 32, 1 << 30, torch.where(d <= 512, 96 // 4, 768 // 4))
+    passes = (quads + tile - 1) // tile
+    u, v = row[:of_roots], col[:of_roots]
+    per_edge = 20 + 32 * octets[v] * (n_low[u] > 0) + 16 * quads[v] * passes[u]
+    return int((per_edge * (d[u] >= 2)).sum())
+
+
 def run_ours(args, world, rank, local, pg):
     import torch
 
@@ -372,14 +418,13 @@ def run_ours(args, world, rank, local, pg):
         peak, peak_src = 6800.0, "fallback"
     kernel_avg_ms = sum(kernel_ms) / len(kernel_ms) if kernel_ms else ms
     sec = kernel_avg_ms / 1000.0
-    # a graph with no row longer than 8 is counted by one flat kernel that
-    # intersects every oriented edge directly (W+ probes, exactly B_alg)
-    flat = launches_per_count == 1
-    probes = W if flat else P_min
-    # the bytes this design must read: each root's row_ptr and list, each
-    # oriented edge's row_ptr pair and the cheaper side's list (every N+(v)
-    # for the flat kernel)
-    B_min = 4 * (V + 1) + 12 * E + 4 * probes + 8
+    kernel = counting_kernel(launches_per_count, int(dplus.max(initial=0)))
+    # the bytes that the kernel must read: the one-launch counts every N+(v), as
+    # plain ids; the tables each root's row_ptr and list, each oriented edge's
+    # row_ptr pair and the cheaper side's list; the packed count its entries
+    probes = P_min if kernel == "count_kernel" else W
+    B_min = (packed_bytes(rp, col, V, dev) if kernel == "packed_kernel" else
+             4 * (V + 1) + 12 * E + 4 * probes + 8)
     tr = load_traffic(cfg["workload"])
     traffic = (tr or {}).get("traffic_bytes_per_launch")
 
@@ -405,14 +450,14 @@ def run_ours(args, world, rank, local, pg):
                     "gpu_launches": (launches_per_count + 2) * args.steps},
             "roofline": {"bound": "hbm", "achieved": B_min / sec / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": B_min / sec / 1e9 / peak, "peak_source": f"{peak_src} hbm_gbs (copy, burst)",
-                         "kernel": (("flat4_kernel" if int(dplus.max(initial=0)) <= 4 else "flat_kernel") if flat
-                                    else "packed_kernel"), "kernel_ms": kernel_avg_ms,
+                         "kernel": kernel, "kernel_ms": kernel_avg_ms,
                          "algorithmic_bytes_per_launch": B_min,
                          "algorithmic_bytes_definition": (
-                             "4(V+1) + 12|E+| + 4 W+ + 8 (the flat kernel probes every wedge)" if flat else
+                             PACKED_BYTES if kernel == "packed_kernel" else
                              "4(V+1) + 12|E+| + 4 sum_{u->v} min(d+(u), d+(v)) + 8: each root's row_ptr and list, "
                              "each oriented edge's row_ptr pair and the cheaper side's list of plain ids "
-                             f"({P_min / max(W, 1):.2f} W+ on this graph; the packed count reads every list, packed)"),
+                             f"({P_min / max(W, 1):.2f} W+ on this graph)" if kernel == "count_kernel" else
+                             "4(V+1) + 12|E+| + 4 W+ + 8 (every wedge is probed)"),
                          "probes_done": probes,
                          "dram_achieved": traffic / sec / 1e9 if traffic else None,
                          "dram_frac": traffic / sec / 1e9 / peak if traffic else None,
@@ -546,7 +591,7 @@ def _part_bytes(prp: np.ndarray, pcol: np.ndarray, n_roots: int) -> tuple[int, i
     model = 4(R+1) + 12 E_R + 4 W+ + 8: the roots' row_ptr and lists, each
     root edge u -> v's row_ptr pair and all of N+(v) (W+ = sum d+(v));
     min-side: the same with min(d+(u), d+(v)) entries per edge, the list of
-    the cheaper side, which is what this design streams through a hash."""
+    the cheaper side, which is what the plain-id tables stream."""
     d = np.diff(prp).astype(np.int64)
     er = int(prp[n_roots])
     if er == 0:
@@ -735,10 +780,13 @@ def run_parts(args, world, rank, local, pg):
     else:
         peak, peak_src = 6800.0, "fallback"
     B_model = B_min = W_tot = 0
+    kernel = counting_kernel(launches, 1 << 30)
     host_parts = []
     for p in parts:
         prp, pcol = p.download()
         bm, bn, w = _part_bytes(prp, pcol, p.n_roots)
+        if kernel == "packed_kernel":
+            bn = packed_bytes(prp, pcol, p.n_roots, dev)
         B_model, B_min, W_tot = B_model + bm, B_min + bn, W_tot + w
         host_parts.append((prp, pcol, p.n_roots))
     k_ms = mean(b_k) if b_k else ms
@@ -747,12 +795,12 @@ def run_parts(args, world, rank, local, pg):
     sec = k_ms / 1000.0
     roofline = {"bound": "hbm", "achieved": B_min / sec / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": B_min / sec / 1e9 / peak, "traffic": traffic,
-                "peak_source": f"{peak_src} hbm_gbs (copy, burst)", "kernel": "packed_kernel of the batched k = 8 count",
+                "peak_source": f"{peak_src} hbm_gbs (copy, burst)", "kernel": f"{kernel} of the batched k = 8 count",
                 "kernel_ms": k_ms, "algorithmic_bytes_per_launch": B_min,
-                "algorithmic_bytes_definition": "sum over parts of 4(R+1) + 12 E_R + 4 sum_{u->v} min(d+(u), d+(v)) "
+                "algorithmic_bytes_definition": f"sum over parts of {PACKED_BYTES}" if kernel == "packed_kernel" else
+                                                "sum over parts of 4(R+1) + 12 E_R + 4 sum_{u->v} min(d+(u), d+(v)) "
                                                 "+ 8 (R roots, E_R root edges): each root's row_ptr and list, each "
-                                                "root edge's row_ptr pair and the cheaper side's list of plain "
-                                                "ids (the packed count reads every list, packed)",
+                                                "root edge's row_ptr pair and the cheaper side's list of plain ids",
                 "dram_achieved": traffic / sec / 1e9 if traffic else None,
                 "dram_frac": traffic / sec / 1e9 / peak if traffic else None,
                 "traffic_source": (tr or {}).get("source"),
@@ -918,8 +966,11 @@ def run_batch(args, world, rank, local, pg):
     e2e_ms = _timed(stream, flush, e2e_call, args.steps, args.warmup)
     clk = clocks.stop()
     B_min = B_model = 0
+    kernel = counting_kernel(b.stats()["launches"], 1 << 30)
     for rp, cl in host:
         bm, bn, _ = _part_bytes(rp, cl, len(rp) - 1)
+        if kernel == "packed_kernel":
+            bn = packed_bytes(rp, cl, len(rp) - 1, dev)
         B_model, B_min = B_model + bm, B_min + bn
     peak, peak_src = _peak()
     k_ms = sum(kms[args.warmup:]) / max(1, len(kms[args.warmup:]))
@@ -945,9 +996,11 @@ def run_batch(args, world, rank, local, pg):
            "roofline": {"bound": "hbm", "achieved": B_min / (k_ms / 1000.0) / 1e9, "peak": peak, "unit": "GB/s",
                         "frac": B_min / (k_ms / 1000.0) / 1e9 / peak, "traffic": None,
                         "peak_source": f"{peak_src} hbm_gbs (copy, burst)",
-                        "kernel": "packed_kernel (batched, 256 graphs)", "kernel_ms": k_ms,
+                        "kernel": f"{kernel} (batched, 256 graphs)", "kernel_ms": k_ms,
                         "algorithmic_bytes_per_launch": B_min,
-                        "algorithmic_bytes_definition": "sum over graphs of 4(V+1) + 12|E+| + 4 sum_{u->v} "
+                        "algorithmic_bytes_definition": f"sum over graphs of {PACKED_BYTES}"
+                                                        if kernel == "packed_kernel" else
+                                                        "sum over graphs of 4(V+1) + 12|E+| + 4 sum_{u->v} "
                                                         "min(d+(u), d+(v)) + 8",
                         "wedge_model_bytes": B_model,
                         "wedge_model_frac": B_model / (k_ms / 1000.0) / 1e9 / peak},

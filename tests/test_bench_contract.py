@@ -86,3 +86,43 @@ def test_gpu_arm_partitioned_line_is_complete():
     assert e2e["value"] > 0 and e2e["h2d_bytes_per_step"] > 0 and e2e["d2h_bytes_per_step"] > 0
     assert d["gpu_launches"] > 0 and "sm_mhz" in d["clocks"]
     assert d["cpu_baseline"]["count_matches"] is True
+
+
+def test_counting_kernel_is_named_by_what_ran():
+    sys.path.insert(0, ROOT)
+    import bench
+    assert [bench.counting_kernel(1, d) for d in (0, 4, 5, 8, 9, 64)] == \
+        ["flat4_kernel"] * 2 + ["flat_kernel"] * 2 + ["single_kernel"] * 2
+    assert bench.counting_kernel(5, 100) == "packed_kernel"
+    assert [bench.counting_kernel(n, 100) for n in (6, 7, 9, 11)] == ["count_kernel"] * 4
+
+
+def test_packed_bytes_of_small_graphs():
+    """By hand, every id of a low block.  K_4 of ids 0..3 (rows of 3, 2, 1 and 0):
+    the roots of two or more members have five out-neighbours, three of them with
+    members, each a row of one octet."""
+    import numpy as np
+    import torch
+    sys.path.insert(0, ROOT)
+    import bench
+    rp, col = np.array([0, 3, 5, 6, 6], np.int32), np.array([1, 2, 3, 2, 3, 3], np.int32)
+    assert bench.packed_bytes(rp, col, 4, torch.device("cpu")) == 5 * 20 + 3 * 32
+    assert bench.packed_bytes(rp, col, 1, torch.device("cpu")) == 3 * 20 + 2 * 32
+    assert bench.packed_bytes(rp, col, 0, torch.device("cpu")) == 0
+    # every id popular once: 40,000 members in rows of one, the first 30,720 ids low
+    n = 40_001
+    rp = np.concatenate(([0, 40_000], np.full(n - 1, 40_000))).astype(np.int32)
+    got = bench.packed_bytes(rp, np.arange(1, n, dtype=np.int32), n, torch.device("cpu"))
+    assert got == 40_000 * 20
+
+
+@pytest.mark.gpu
+def test_roofline_names_the_kernel_that_counted():
+    """R-MAT 16 counts packed, a road network flat, an unskewed batch's or the probing tables' count by count_kernel."""
+    for extra, kernel in ((["--workload", "rmat16", "--no-tune"], "packed_kernel"),
+                          (["--workload", "rmat16", "--tuning", '{"probe_kicks": 0}'], "count_kernel")):
+        out = subprocess.run([sys.executable, "bench.py", "--steps", "2", "--warmup", "3", "--no-cpu"] + extra,
+                             cwd=ROOT, capture_output=True, text=True, timeout=900, check=True).stdout
+        d = json.loads([line for line in out.splitlines() if line.startswith("{")][0])
+        assert d["roofline"]["kernel"] == kernel
+        assert (d["roofline"]["probes_done"] == d["config"]["W_plus"]) == (kernel == "packed_kernel")
