@@ -8,14 +8,15 @@
 // entries of the renumbered ids: entry = (block << mbits) | mask, bit i of the
 // mask standing for id block * mbits + i.  Popular ids are in most lists and
 // sit together, so a list's many popular ids share few entries (R-MAT 20:
-// 0.81 entries per id over all rows, but 0.41 x the ids along the lists that
+// 0.81 entries per id over all rows, but 0.37 x the ids along the lists that
 // the count streams), and the blocks that a probe looks for are mostly small
-// numbers: 97 % of R-MAT 20's streamed entries have a block below 4096.  So
-//   * a root's row is a table addressed by the block itself for blocks < D
+// numbers: 99 % of R-MAT 20's streamed entries are of the first 2048 blocks
+// (kLow).  So
+//   * a root's row is a table addressed by the block itself for blocks < kLow
 //     (one 16-bit shared load per probe; a list's blocks ascend there, so a
 //     warp's 32 loads fall in neighbouring words), with a small linear-probing
 //     hash for the rest;
-//   * a probe is one AND and one popcount for up to 16 ids.
+//   * a probe is one AND and half a popcount for up to 15 ids.
 // Every root streams the lists of all its out-neighbours through its own table
 // (W+ ids in the reference's terms).  Compared with choosing the shorter side
 // per edge that is 1.0-2.4 x the entries, but there is no transpose of the
@@ -939,10 +940,11 @@ __device__ __noinline__ uint32_t self_member(const Rows<false> &R, int v, const 
 // that find no more of one kind fill the others' tail.  Bound by the L1 / shared
 // pipe and by issue: a warp's round is two 16-byte loads of entries per lane and
 // eight look-ups, about 100 instructions per 256 entries.  R-MAT 21, whole:
-// 17.9 G W+ probes are 4.2 G entries; 2.9 ms against 6.0 for the plain-id tables
-// (6.68 -> 3.5 ms per count with the passes before).  4 blocks per SM (64
-// registers): with 5 (48) the next round's loads do not fit beside this
-// round's, 4.3 instead of 3.8 ms.
+// 11.3 G W+ probes are 4.4 G entries; 2.45 ms against 5.98 for the plain-id tables
+// (6.68 -> 2.88 ms per count with the passes before): the pipe 88 % busy, 61 % of
+// the issue slots, 8.6 TB/s from L2.  4 blocks per SM (64 registers): with 5 (48)
+// the next round's loads did not fit beside this round's, 4.3 instead of the 3.8 ms
+// that it took then.
 constexpr int kPackedMinBlocks = 4;
 template <bool kPerRoot>
 __global__ void __launch_bounds__(kThreads, kPackedMinBlocks) packed_kernel(PackParams P) {

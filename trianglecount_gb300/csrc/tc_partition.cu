@@ -17,7 +17,8 @@
 //            room left under the cap ceil(1.03 n / k) plus the candidates
 //            expected to leave b, W_b: candidates for b), decided by a seeded
 //            hash; part sizes are recounted
-// until fewer than 0.1% of the vertices move or the iteration budget is spent.
+// until fewer than 0.1% of the vertices move or the iteration budget is spent
+// (looked at from the host after two iterations, then after every eight).
 // Measured cut fractions at k = 8 (random parts: 0.875): Chung-Lu 0.71,
 // R-MAT 0.81 (its hubs touch every part), a road grid 0.002; largest part
 // 1.03 x the mean.
@@ -31,7 +32,7 @@ namespace {
 
 constexpr int kMaxParts = 64;
 constexpr int kPT = 256;  // threads per block
-constexpr int kLpFlight = 4;  // neighbours per lane and round (two: 1.37 instead of 1.31 ms)
+constexpr int kLpFlight = 4;  // neighbours per lane and round (two: 1.37 instead of 1.31 ms then)
 constexpr int kGroupDeg = 255, kAloneDeg = 64, kWarpDeg = 1024;  // see lp_choose_kernel
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -122,7 +123,7 @@ __device__ __forceinline__ int lp_pick(const int32_t *h, int k, uint64_t seed, i
 // summed over the lanes with shuffles -- no histogram in memory, and the warp
 // waits for four vertices' gathers at once.  (One warp per vertex with a shared
 // histogram left most lanes idle on most rows: Chung-Lu n = 500 K, mean degree
-// 16, k = 8, 20 iterations 4.00 ms the whole call, 1.31 ms so.)  With more parts
+// 16, k = 8, 20 iterations 3.87 ms the whole call, 1.26 ms so.)  With more parts
 // vertices of degree <= 64 (kAloneDeg) are counted one at a time in the warp's
 // histogram.  A warp takes per_warp consecutive vertices of these: 32, or fewer
 // while that many would leave SMs without a block (lp_per_warp).  The others come
