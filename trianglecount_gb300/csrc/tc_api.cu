@@ -27,7 +27,7 @@ struct ValidateErr {
     int first;      // smallest offending row / entry index
     RowStats rows;  // of valid rows
 };
-constexpr ValidateErr kNoErr{0, 0x7fffffff, {0, 0, 0}};
+constexpr ValidateErr kNoErr{0, 0x7fffffff, {0, 0, 0, 0}};
 
 __global__ void mark_rows_kernel(const int32_t *rp, int64_t n_rows, int64_t nnz, RowBounds bounds, uint8_t *start,
                                  ValidateErr *err) {
@@ -272,27 +272,33 @@ bool flat_count(const tc_graph *g) {
 // so does a launch with as many of its entries in such graphs.
 //   Every row is packed, also the rows that no root holds, and every row, empty or
 // not, is looked at by four passes: a few roots of a large graph, or few edges
-// among many rows, do not pay for that.  R-MAT 20 (16 M edges) counts 0.12 / 0.48 /
-// 1.2 M root edges in 0.35 / 0.31 / 0.36 ms packed, 0.25 / 0.35 / 0.51 plain;
-// Chung-Lu n = 1 M (8 M edges) 0.39 / 0.79 M in 0.25 / 0.26 and 0.22 / 0.27;
-// R-MAT 16 (0.9 M edges) in 4 / 8 M rows 0.28 / 0.48 and 0.33 / 0.39, R-MAT 19
-// (7.7 M) in 16 / 32 M rows 1.24 / 2.07 and 1.68 / 1.98.  Graphs of any of these
-// shapes with fewer than 2^18 edges and rows gain from the fewer launches.
-constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440, kPackFree = 1 << 18;
+// among many rows, do not pay for that.  From such launches' times, the packed count
+// saves about 50 us (fewer launches) and 200 ps per root edge, and costs 5 ps per
+// entry, 190 ps per row that has any and 48 per row that has none (pays).  R-MAT 20
+// (16 M edges) counts 0.25 / 0.48 / 1.2 M root edges in 0.32 / 0.31 / 0.36 ms packed,
+// 0.29 / 0.35 / 0.51 plain; Chung-Lu n = 1 M (8 M edges) 0.39 / 2.4 M in 0.25 /
+// 0.33 and 0.22 / 0.44; R-MAT 16 (0.9 M edges) in 4 / 8 M rows 0.28 / 0.48 and 0.33 /
+// 0.39; R-MAT 20's 64 halo parts (497 M edges, 16 M of them the roots') 4.9 and 6.8.
+//   A batch of tiny graphs pays for each graph in the passes that rank its ids: 8000
+// graphs of 62 / 559 / 3448 edges 0.26 / 0.41 / 1.31 ms packed, 0.13 / 0.35 / 1.70
+// plain, 100 of 559 0.08 and 0.10.
+constexpr int64_t kSkewShare = 16, kFarShare = 16, kPackRows = 61440, kTinyEdges = 1536, kTinyFree = 1 << 16;
 bool skewed(const tc_graph *g) { return g->rows.longest >= 0 && kSkewShare * g->rows.skewed >= g->nnz; }
 bool far_rows(const tc_graph *g) { return g->rows.far > 0 && kFarShare * g->rows.far >= g->nnz; }
 bool packed_graphs(const tc_graph *const *gs, int n, const Tuned &tn) {
     if (!packed_count(tn)) return false;
-    int64_t V = 0, E = 0, gain = 0, far = 0, of_roots = kPackFree;
+    int64_t V = 0, E = 0, gain = 0, far = 0, of_roots = 0, filled = 0;
     for (int i = 0; i < n; ++i) {
         const tc_graph *g = gs[i];
         if (g->n_rows > kPackRows && far_rows(g)) far += g->nnz;
         else if (g->n_rows <= kPackRows || skewed(g)) gain += g->nnz;
         if (g->root_nnz >= 0) of_roots += g->root_nnz;
+        filled += g->rows.filled;
         V += g->n_rows + 1;
         E += g->nnz;
     }
-    return 2 * gain >= E && kFarShare * far <= E && of_roots >= E / 16 + V / 4 && pack_fits(V, E);
+    const bool pays = 50'000'000 + 200 * of_roots >= 5 * E + 190 * filled + 48 * (V - filled);  // ps
+    return 2 * gain >= E && kFarShare * far <= E && pays && kTinyEdges * n <= E + kTinyFree && pack_fits(V, E);
 }
 bool packed_graph(const tc_graph *g) { return !g->no_pack && packed_graphs(&g, 1, g->ctx->tuned); }
 

@@ -252,6 +252,7 @@ struct RowStats {
     int32_t longest = -1;  // the longest row; -1: not known
     uint32_t skewed = 0;   // entries in rows longer than kSkew x the mean
     uint32_t far = 0;      // entries in rows that no degree orientation has (RowBounds)
+    int32_t filled = 0;    // rows that have entries
 };
 // An orientation by degree has rows of at most sqrt(2 nnz) members, and in R-MAT
 // and Chung-Lu graphs of at most a tenth of that.
@@ -282,24 +283,25 @@ __device__ __forceinline__ void push_together(int32_t *list, int32_t *n, int32_t
 // halo extraction, 30 us of its 1 ms).
 struct RowTally {
     int longest = 0;
-    unsigned skewed = 0, far = 0, of_roots = 0;
+    unsigned skewed = 0, far = 0, filled = 0, of_roots = 0;
     __device__ __forceinline__ void row(int d, RowBounds b) {
         longest = max(longest, d);
+        filled += (unsigned)(d > 0);
         if (d > b.skew) skewed += (unsigned)d;
         if (d > b.far) far += (unsigned)d;
     }
     __device__ __forceinline__ void add(RowStats *out, int32_t *root_nnz = nullptr) {
         __shared__ int s_longest;
-        __shared__ unsigned s_sum[3];
-        if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+        __shared__ unsigned s_sum[4];
+        if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
         if (threadIdx.x == 0) s_longest = 0;
         __syncthreads();
         longest = __reduce_max_sync(0xffffffffu, longest);
-        const unsigned sum[3] = {__reduce_add_sync(0xffffffffu, skewed), __reduce_add_sync(0xffffffffu, far),
-                                 __reduce_add_sync(0xffffffffu, of_roots)};
+        const unsigned sum[4] = {__reduce_add_sync(0xffffffffu, skewed), __reduce_add_sync(0xffffffffu, far),
+                                 __reduce_add_sync(0xffffffffu, of_roots), __reduce_add_sync(0xffffffffu, filled)};
         if ((threadIdx.x & 31) == 0 && longest) {
             atomicMax(&s_longest, longest);
-            for (int i = 0; i < 3; ++i)
+            for (int i = 0; i < 4; ++i)
                 if (sum[i]) atomicAdd(&s_sum[i], sum[i]);
         }
         __syncthreads();
@@ -308,6 +310,7 @@ struct RowTally {
             if (s_sum[0]) atomicAdd(&out->skewed, s_sum[0]);
             if (s_sum[1]) atomicAdd(&out->far, s_sum[1]);
             if (root_nnz && s_sum[2]) atomicAdd(root_nnz, (int)s_sum[2]);
+            atomicAdd(&out->filled, (int)s_sum[3]);
         }
     }
 };
