@@ -450,12 +450,13 @@ __global__ void __launch_bounds__(kThreads, 5) pack_kernel(PackParams P) {
                 int i = at + warp_excl_scan(__popc(f), lane, &tot);
                 at += tot;
                 if (tot == 0) continue;
-                if (f) *d4 = make_uint4(0, 0, 0, 0);
-                for (; f; f &= f - 1u) {  // the masks from v: dir's words are not read again as halves of them
-                    const int j = __ffs(f) - 1;
-                    const uint32_t pair = j & 4 ? (j & 2 ? v.w : v.z) : (j & 2 ? v.y : v.x);
-                    lrow[deal(i++)] = ((uint32_t)(8 * w + j) << 16) | (j & 1 ? pair >> 16 : pair & 0xffffu);
+                const bool any = f != 0;
+                for (; f; f &= f - 1u) {
+                    const int b = 8 * w + __ffs(f) - 1;
+                    lrow[deal(i++)] = ((uint32_t)b << 16) | reinterpret_cast<const uint16_t *>(dir)[b];
                 }
+                asm volatile("" ::: "memory");  // halves are read, whole words cleared: not to be taken for others
+                if (any) *d4 = make_uint4(0, 0, 0, 0);
             }
             for (int w = lane; w < n_list; w += kWarp) {
                 const int b = s_list[warp][w];
