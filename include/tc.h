@@ -161,7 +161,9 @@ TC_API int tc_graph_upload_i32(tc_ctx *ctx, const int32_t *row_ptr, const int32_
                                int64_t nnz, int64_t n_roots, tc_graph **out);
 TC_API int tc_graph_upload_u64(tc_ctx *ctx, const uint64_t *row_ptr, const uint64_t *col, int64_t n_rows,
                                int64_t nnz, int64_t n_roots, tc_graph **out);
-/* Wrap caller-owned device arrays without copying (no validation). */
+/* Wrap caller-owned device arrays without copying (no validation).  The first
+ * count that waits for its result, or tc_batch_create, also reads d_row_ptr to
+ * choose the count; the arrays may hold another graph of the same sizes later. */
 TC_API int tc_graph_wrap_device_i32(tc_ctx *ctx, const int32_t *d_row_ptr, const int32_t *d_col, int64_t n_rows,
                                     int64_t nnz, int64_t n_roots, tc_graph **out);
 TC_API int tc_graph_info(const tc_graph *g, int64_t *n_rows, int64_t *nnz, int64_t *n_roots);

@@ -686,7 +686,7 @@ int device_sm_count(int device) {
 int row_stats(tc_ctx *ctx, const int32_t *rp, int64_t n_rows, int64_t nnz, RowStats *d_out) {
     TC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(RowStats), ctx->stream));
     if (n_rows > 0)
-        row_stats_kernel<<<grid_for(n_rows, ctx->sm_count), 256, 0, ctx->stream>>>(rp, n_rows, row_bounds(n_rows, nnz),
+        row_stats_kernel<<<std::min(grid_for(n_rows, ctx->sm_count), ctx->sm_count * 8), 256, 0, ctx->stream>>>(rp, n_rows, row_bounds(n_rows, nnz),
                                                                                    d_out);
     TC_CUDA(cudaGetLastError());
     return TC_OK;

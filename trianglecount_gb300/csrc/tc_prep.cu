@@ -1016,7 +1016,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
             TC_CUDA(cudaMemsetAsync(lrp.p, 0, sizeof(int32_t) * ((size_t)V + 1), s));
             TC_CUDA(cudaMemsetAsync(&words.p->root_nnz, 0, sizeof(HaloWords) - offsetof(HaloWords, root_nnz), s));
             if (V)
-                halo_ids_kernel<<<gV, 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, row_bounds(V, nnz / 2),
+                halo_ids_kernel<<<std::min(gV, ctx->sm_count * 8), 256, 0, s>>>(cd.p, removed.p, ids.p, cnt.p, V, lid.p, lrp.p, row_bounds(V, nnz / 2),
                                                    words.p);
             TC_CUDA(cudaGetLastError());
             TC_TRY(scan_exclusive_i32(lrp.p, lrp.p, V, s));  // rows past the part's are empty
@@ -1034,7 +1034,7 @@ int tc_halo_extract_ex(tc_ctx *ctx, const tc_ugraph *ug, const int32_t *part, in
         TC_TRY(number());
         TC_TRY(look());
         if (!in_only && back->words.front[round % 3] != 0) {
-            for (int more = 8; back->words.front[round % 3] != 0; more = std::min(64, 2 * more)) {
+            for (int more = 4; back->words.front[round % 3] != 0; more = std::min(64, 2 * more)) {
                 peel(more);
                 TC_CUDA(cudaGetLastError());
                 TC_TRY(look());
