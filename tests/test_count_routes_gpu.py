@@ -2,10 +2,13 @@
 The packed count is five launches; the plain-id count of more than 4096 rows at
 least seven (its scan alone takes three).  Every count is also checked against
 the oracle, on either side of each rule."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import oracle
+import trianglecount_gb300 as tc
 from trianglecount_gb300 import generators as gen
 
 pytestmark = pytest.mark.gpu
@@ -44,9 +47,33 @@ def launches_of(ctx, rp, col, n_roots=None):
     g = ctx.upload(rp, col, n_roots=n_roots)
     got, st = ctx.count(g, stats=True)
     assert got == want
-    assert np.array_equal(ctx.count_per_root(g), pr)
+    assert per_root_and_total(ctx, g, pr) == want
     assert list(ctx.batch([g]).run()) == [want]
     return st["launches"]
+
+
+def per_root_and_total(ctx, g, want):
+    """Checks the per-root counts; the total that the call gives beside them."""
+    got, total = np.full(len(want), 7, np.uint64), ctypes.c_uint64()
+    st = tc.lib().tc_count_per_root(ctx.handle, g.handle, got.ctypes.data_as(ctypes.c_void_p), ctypes.byref(total))
+    assert st == 0 and np.array_equal(got, want)
+    return total.value
+
+
+@pytest.mark.parametrize("self_loops", [False, True])
+def test_total_beside_the_per_root_counts(ctx, self_loops):
+    """Flat rows of up to 4 and 8, one launch, packed and plain-id tables, all rows and a prefix of them as roots."""
+    r = np.random.default_rng(3)
+    for n, most in ((5000, 4), (5000, 8), (5000, 40), (60_000, 60), (100_000, 20)):
+        u = np.repeat(np.arange(n), r.integers(0, most + 1, n))
+        v = r.integers(0, n, len(u)) % max(1, n // 8) if most < 20 else r.integers(0, n, len(u))
+        if not self_loops:
+            u, v = u[u != v], v[u != v]
+        elif most > 4:
+            u, v = np.concatenate((u, np.arange(0, n, 7))), np.concatenate((v, np.arange(0, n, 7)))
+        rp, col = csr(n, u, v)
+        for n_roots in (None, n // 3):
+            launches_of(ctx, rp, col, n_roots)
 
 
 def test_one_clique_does_not_make_a_graph_skewed(ctx):
@@ -189,7 +216,6 @@ def wrapped(ctx, rp, col):
 
 def count_async(ctx, g):
     import torch
-    import trianglecount_gb300 as tc
     out = torch.zeros(1, dtype=torch.int64, device="cuda")
     torch.cuda.synchronize()
     assert tc.lib().tc_count_async(ctx.handle, g.handle, out.data_ptr()) == 0
@@ -239,7 +265,6 @@ def test_wrapped_arrays_may_be_written_anew(ctx):
 def test_a_callers_capture_outlives_the_look_at_the_rows():
     """tc_count_async captured by the caller, then a count that takes another form: the capture still counts."""
     torch = pytest.importorskip("torch")
-    import trianglecount_gb300 as tc
     rp, col, want = oracle.pipeline(*gen.rmat(17))
     c = tc.Context(0)
     s = torch.cuda.Stream()
